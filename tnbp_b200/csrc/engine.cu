@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "../../include/tnbp_b200.h"
+#include "dmma.cuh"
 #include "engine.h"
 #include "host_setup.h"
 #include "kernels.cuh"
@@ -993,7 +994,8 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
   // tcgen05 kernel, every other task on the CUDA-core kernel, whatever else
   // shares the batch.  A request's rounding therefore does not depend on
   // what it is batched with.
-  const bool tc_ok = !entries.empty() && reduced_sweeps(entries[0].job->prec) && tcgen05_enabled();
+  const bool reduced = !entries.empty() && reduced_sweeps(entries[0].job->prec);
+  const bool tc_ok = reduced && tcgen05_enabled();
   {
     // small sites: one CTA each, every message of the site on chip
     std::vector<SiteTask> sts;
@@ -1036,7 +1038,7 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
           } else {
             lt.block_begin = nb;
             beg.push_back(nb);
-            nb += (lt.L * lt.R + kRowTile - 1) / kRowTile;
+            nb += reduced ? (lt.L * lt.R + kRowTile - 1) / kRowTile : dm::leg_tiles(lt.L, lt.R);
             maxdin = std::max(maxdin, lt.Din);
             t.push_back(lt);
           }
@@ -1121,10 +1123,27 @@ static void leg_apply_attr() {
   static std::vector<char> flags;
   std::lock_guard<std::mutex> lk(g_attr_mu);
   if (attr_done(flags)) return;
-  CK(cudaFuncSetAttribute(k_leg_apply<R, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)leg_smem<R>(128)));
+  if constexpr (sizeof(R) == 8) {
+    CK(cudaFuncSetAttribute(k_leg_apply_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dm::leg_smem_bytes(128)));
+    CK(cudaFuncSetAttribute(k_gram_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dm::gram_smem_bytes()));
+  } else {
+    CK(cudaFuncSetAttribute(k_leg_apply<R, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)leg_smem<R>(128)));
+  }
   CK(cudaFuncSetAttribute(k_site_sweep<R, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSiteSmemMax));
   attr_mark(flags);
 }
+
+// The FP64 kernels of dmma.cuh live in this translation unit, where
+// prepare_kernels raises their shared memory limits.
+void launch_leg_f64(const LegTask* tasks, const long long* begins, int ntask, long long nblocks, int max_din,
+                    cudaStream_t stream) {
+  k_leg_apply_f64<<<(unsigned)nblocks, dm::kLegThreads, dm::leg_smem_bytes(max_din), stream>>>(tasks, begins, ntask,
+                                                                                              max_din);
+}
+void launch_gram_f64(const GramTask* tasks, const long long* begins, int ntask, long long nblocks, cudaStream_t stream) {
+  k_gram_f64<<<(unsigned)nblocks, dm::kGramThreads, dm::gram_smem_bytes(), stream>>>(tasks, begins, ntask);
+}
+long long leg_tiles_f64(long long L, long long R) { return dm::leg_tiles(L, R); }
 
 template <typename R, typename MR>
 static int launch_batch_t(const SweepBatch& b, cudaStream_t stream) {
@@ -1156,8 +1175,11 @@ static int launch_batch_t(const SweepBatch& b, cudaStream_t stream) {
       }
       case SweepLaunch::LEG_CORE: {
         if (L.max_din > 128) throw Error(TNBP_EUNSUPPORTED, "bond dimension above 128 during BP");
-        k_leg_apply<R, MR><<<(unsigned)L.nblocks, kThreads, leg_smem<R>(L.max_din), stream>>>(
-            static_cast<const LegTask*>(tasks), begins, L.ntask, L.max_din);
+        if constexpr (sizeof(R) == 8)
+          launch_leg_f64(static_cast<const LegTask*>(tasks), begins, L.ntask, L.nblocks, L.max_din, stream);
+        else
+          k_leg_apply<R, MR><<<(unsigned)L.nblocks, kThreads, leg_smem<R>(L.max_din), stream>>>(
+              static_cast<const LegTask*>(tasks), begins, L.ntask, L.max_din);
         break;
       }
       case SweepLaunch::GRAM_TC:
@@ -1173,7 +1195,10 @@ static int launch_batch_t(const SweepBatch& b, cudaStream_t stream) {
             static_cast<const LegGramTask*>(tasks), begins, L.ntask);
         break;
       case SweepLaunch::GRAM_CORE:
-        k_gram<R><<<(unsigned)L.nblocks, kThreads, 0, stream>>>(static_cast<const GramTask*>(tasks), begins, L.ntask);
+        if constexpr (sizeof(R) == 8)
+          launch_gram_f64(static_cast<const GramTask*>(tasks), begins, L.ntask, L.nblocks, stream);
+        else
+          k_gram<R><<<(unsigned)L.nblocks, kThreads, 0, stream>>>(static_cast<const GramTask*>(tasks), begins, L.ntask);
         break;
       case SweepLaunch::MSG:
         k_msg_finalize<R, MR><<<L.ntask, kThreads, 0, stream>>>(static_cast<const MsgTask*>(tasks));
@@ -1592,7 +1617,7 @@ void Job::run_chains(std::vector<ChainEntry>& chains) {
         set_leg_divisors(lt);
         lt.block_begin = nb;
         b.push_back(nb);
-        nb += (L * R + kRowTile - 1) / kRowTile;
+        nb += sprec == TNBP_C128 ? dm::leg_tiles(L, R) : (L * R + kRowTile - 1) / kRowTile;
         maxdin = std::max(maxdin, lt.Din);
         t.push_back(lt);
       }
@@ -1602,8 +1627,8 @@ void Job::run_chains(std::vector<ChainEntry>& chains) {
       if (maxdin > 128) throw Error(TNBP_EUNSUPPORTED, "bond dimension above 128");
       prepare_kernels(sprec);
       if (sprec == TNBP_C128) {
-        const size_t smem = leg_smem<double>(maxdin);
-        (k_leg_apply<double><<<(unsigned)nb, kThreads, smem, stream>>>(static_cast<LegTask*>(dt.p), static_cast<long long*>(db.p), (int)t.size(), maxdin), note_launch());
+        launch_leg_f64(static_cast<LegTask*>(dt.p), static_cast<long long*>(db.p), (int)t.size(), nb, maxdin, stream);
+        note_launch();
       } else {
         const size_t smem = leg_smem<float>(maxdin);
         (k_leg_apply<float><<<(unsigned)nb, kThreads, smem, stream>>>(static_cast<LegTask*>(dt.p), static_cast<long long*>(db.p), (int)t.size(), maxdin), note_launch());
@@ -1875,7 +1900,8 @@ void Job::env_grams(const std::vector<EnvReq>& reqs, DevBuf& out, std::vector<si
   upload_vec(dgb, gb, stream);
   upload_vec(dpt, pt, stream);
   if (!gt.empty()) {
-    if (sprec == TNBP_C128) (k_gram<double><<<(unsigned)nb, kThreads, 0, stream>>>(static_cast<GramTask*>(dgt.p), static_cast<long long*>(dgb.p), (int)gt.size()), note_launch());
+    prepare_kernels(sprec);
+    if (sprec == TNBP_C128) (launch_gram_f64(static_cast<GramTask*>(dgt.p), static_cast<long long*>(dgb.p), (int)gt.size(), nb, stream), note_launch());
     else (k_gram<float><<<(unsigned)nb, kThreads, 0, stream>>>(static_cast<GramTask*>(dgt.p), static_cast<long long*>(dgb.p), (int)gt.size()), note_launch());
     CK(cudaGetLastError());
     (k_partial_sum<<<(unsigned)pt.size(), kThreads, 0, stream>>>(static_cast<PartialSumTask*>(dpt.p)), note_launch());

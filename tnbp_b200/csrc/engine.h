@@ -143,6 +143,10 @@ double effective_tol(int prec, double tol);
 bool stop_on_growth(int prec, double prev, double c);
 inline bool reduced_sweeps(int prec) { return prec != TNBP_C128; }
 void prepare_kernels(int prec);
+void launch_leg_f64(const LegTask* tasks, const long long* begins, int ntask, long long nblocks, int max_din,
+                    cudaStream_t stream);
+void launch_gram_f64(const GramTask* tasks, const long long* begins, int ntask, long long nblocks, cudaStream_t stream);
+long long leg_tiles_f64(long long L, long long R);
 size_t wave_budget_bytes();
 size_t scratch_cap_bytes();
 size_t device_bytes_available();

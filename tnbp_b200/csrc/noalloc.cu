@@ -2,8 +2,8 @@
 //
 // Same arithmetic as one message of the sweep (bp.h:128-175): the site
 // tensor absorbs the incoming messages on every leg but the target
-// (k_leg_apply, one launch per leg), the result is contracted with conj(V)
-// over all legs but the target (k_gram, split-K partials) and the sum is
+// (k_leg_apply_f64, one launch per leg), the result is contracted with conj(V)
+// over all legs but the target (k_gram_f64, split-K partials) and the sum is
 // normalized (k_msg_finalize).  The intermediate tensors, the Gram partials
 // and the task descriptors live in g_noalloc_scratch, a file-scope
 // __device__ array, instead of memory from cudaMalloc/cudaMallocAsync.
@@ -170,13 +170,11 @@ void message_noalloc(const double* site, const int32_t* shape, int32_t rank, int
   prepare_kernels(TNBP_C128);
   for (size_t i = 0; i < legs.size(); ++i) {
     const LegTask& t = legs[i];
-    const long long nb = (t.L * t.R + kRowTile - 1) / kRowTile;
-    const size_t smem = (size_t)(kRowTile * (t.Din + 1) + t.Din * (kColTile + 1)) * sizeof(double2);
-    k_leg_apply<double><<<(unsigned)nb, kThreads, smem, stream>>>(&d_pack->leg[i], d_zero, 1, t.Din);
+    launch_leg_f64(&d_pack->leg[i], d_zero, 1, leg_tiles_f64(t.L, t.R), t.Din, stream);
     CK(cudaGetLastError());
     note_launch(1);
   }
-  k_gram<double><<<(unsigned)((long long)gt.nchunk * gt.ctiles * gt.ctiles), kThreads, 0, stream>>>(d_gram, d_zero, 1);
+  launch_gram_f64(d_gram, d_zero, 1, (long long)gt.nchunk * gt.ctiles * gt.ctiles, stream);
   CK(cudaGetLastError());
   k_msg_finalize<double><<<1, kThreads, 0, stream>>>(d_msg);
   CK(cudaGetLastError());

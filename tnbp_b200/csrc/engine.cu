@@ -746,10 +746,21 @@ void Job::build_plan() {
   }
   // 2. waves of consecutive units within the byte budget (at least one unit)
   if (!tuning) choose_wave_budget();
-  size_t cap = 0;
-  {
+  // A sweep whose slots fit the smallest limit (or the scratch the job
+  // already holds) is one wave whatever the device has left, so only larger
+  // ones ask: the driver's memory query waits on locks shared with other
+  // processes of the machine and took up to 90 ms here (a whole 4x4 chi 4
+  // solve: 4.2 ms without it, 4.3 to 30 ms on average with it).
+  size_t slots = 0, whole = 0;
+  for (const Unit& U : units) {
+    const size_t site_b = align_elems(site_elems(U.site)) * wsz;
+    slots += (size_t)U.nbuf * site_b;
+    whole += (size_t)(U.nbuf + 1) * site_b;
+  }
+  size_t cap = scratch_cap ? scratch_cap : scratch_cap_bytes();
+  if (!scratch_cap && whole > cap) {
     TNBP_TRACE_SCOPE("sweep.build_plan.scratch_limit");
-    cap = scratch_limit();
+    cap = slots <= ws_scratch.bytes ? whole : scratch_limit();
   }
   const size_t budget = wave_budget && wave_budget < cap ? wave_budget : cap;
   std::vector<std::vector<int>> waves;

@@ -1652,12 +1652,36 @@ void Job::run_chains(std::vector<ChainEntry>& chains) {
 }
 
 // --------------------------------------------------------------- truncation
+template <typename R>
+static void launch_truncation(const TruncTask* tasks, int ne, int max_d, int chi_max, double sv_min, cudaStream_t stream) {
+  {
+    static std::vector<char> flags;
+    std::lock_guard<std::mutex> lk(g_attr_mu);
+    if (!attr_done(flags)) {
+      const int most = (int)trunc_smem_bytes(kTruncMaxD);
+      CK(cudaFuncSetAttribute(k_trunc_roots<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+      CK(cudaFuncSetAttribute(k_truncate_edges<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+      attr_mark(flags);
+    }
+  }
+  const size_t smem = trunc_smem_bytes(max_d);
+  const int threads = trunc_threads(max_d);
+  k_trunc_roots<R><<<2 * ne, threads, smem, stream>>>(tasks, sv_min, max_d);
+  CK(cudaGetLastError());
+  k_truncate_edges<R><<<ne, threads, smem, stream>>>(tasks, chi_max, sv_min, max_d);
+  CK(cudaGetLastError());
+  note_launch(2);
+}
+
 void Job::truncate(int chi_max, double sv_min, int32_t* dims_out, double* err_out) {
   TNBP_TRACE_SCOPE("truncate");
   shadow_dirty = true;
   if (chi_max < 1) throw Error(TNBP_EINVAL, "chi_max must be >= 1");
   const int ns = (int)g.labels.size();
   const int ne = (int)g.edges.size();
+  int max_d = 1;
+  for (int d : dim) max_d = std::max(max_d, d);
+  if (max_d > kTruncMaxD) throw Error(TNBP_EUNSUPPORTED, "bond dimension above 128");
   // per-edge scratch
   std::vector<size_t> woff(ne), poff(ne), soff(ne);
   size_t wtot = 0, ptot = 0, stot = 0;
@@ -1667,16 +1691,14 @@ void Job::truncate(int chi_max, double sv_min, int32_t* dims_out, double* err_ou
     poff[e] = ptot; ptot += align_elems(nn);
     soff[e] = stot; stot += (size_t)dim[e];
   }
-  DevBuf work, sv, perm, Pa, Pb, skeep, keep, err, status;
+  DevBuf work, Pa, Pb, skeep, keep, err, status;
   work.alloc(wtot * sizeof(double2), stream);
-  sv.alloc(3 * stot * sizeof(double), stream);
-  perm.alloc(3 * stot * sizeof(int), stream);
   Pa.alloc(ptot * esz, stream);
   Pb.alloc(ptot * esz, stream);
   skeep.alloc(stot * sizeof(double), stream);
   keep.alloc(ne * sizeof(int), stream);
   err.alloc(ne * sizeof(double), stream);
-  status.alloc(ne * sizeof(int), stream);
+  status.alloc(3 * ne * sizeof(int), stream);
   std::vector<TruncTask> tt(ne);
   for (int e = 0; e < ne; ++e) {
     TruncTask& t = tt[e];
@@ -1684,27 +1706,24 @@ void Job::truncate(int chi_max, double sv_min, int32_t* dims_out, double* err_ou
     t.Mb = mptr(cur, e + ne);
     t.D = dim[e];
     t.work = static_cast<double2*>(work.p) + woff[e];
-    t.sv = static_cast<double*>(sv.p) + 3 * soff[e];
-    t.perm = static_cast<int*>(perm.p) + 3 * soff[e];
     t.Pa = static_cast<char*>(Pa.p) + poff[e] * esz;
     t.Pb = static_cast<char*>(Pb.p) + poff[e] * esz;
     t.s_keep = static_cast<double*>(skeep.p) + soff[e];
     t.keep_out = static_cast<int*>(keep.p) + e;
     t.err_out = static_cast<double*>(err.p) + e;
-    t.status = static_cast<int*>(status.p) + e;
+    t.status = static_cast<int*>(status.p) + 3 * e;
   }
   DevBuf dtt;
   upload_vec(dtt, tt, stream);
-  if (sprec == TNBP_C128) (k_truncate_edges<double><<<ne, kThreads, 0, stream>>>(static_cast<TruncTask*>(dtt.p), chi_max, sv_min), note_launch());
-  else (k_truncate_edges<float><<<ne, kThreads, 0, stream>>>(static_cast<TruncTask*>(dtt.p), chi_max, sv_min), note_launch());
-  CK(cudaGetLastError());
-  std::vector<int> hkeep(ne), hstatus(ne);
+  if (sprec == TNBP_C128) launch_truncation<double>(static_cast<TruncTask*>(dtt.p), ne, max_d, chi_max, sv_min, stream);
+  else launch_truncation<float>(static_cast<TruncTask*>(dtt.p), ne, max_d, chi_max, sv_min, stream);
+  std::vector<int> hkeep(ne), hstatus(3 * ne);
   std::vector<double> herr(ne);
   {
     TNBP_TRACE_SCOPE("truncate.svd_wait");
     CK(cudaMemcpyAsync(hkeep.data(), keep.p, ne * sizeof(int), cudaMemcpyDeviceToHost, stream));
     CK(cudaMemcpyAsync(herr.data(), err.p, ne * sizeof(double), cudaMemcpyDeviceToHost, stream));
-    CK(cudaMemcpyAsync(hstatus.data(), status.p, ne * sizeof(int), cudaMemcpyDeviceToHost, stream));
+    CK(cudaMemcpyAsync(hstatus.data(), status.p, 3 * ne * sizeof(int), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
   }
   // new site tensors: V_s x_k P_k for every leg, then normalize
@@ -1768,8 +1787,9 @@ void Job::truncate(int chi_max, double sv_min, int32_t* dims_out, double* err_ou
   if (err_out) for (int e = 0; e < ne; ++e) err_out[e] = herr[e];
   int bad = 0, nonfinite = 0;
   for (int e = 0; e < ne; ++e) {
-    bad += hstatus[e] == 1;
-    nonfinite += hstatus[e] == 2;
+    const int st = std::max(hstatus[3 * e], std::max(hstatus[3 * e + 1], hstatus[3 * e + 2]));
+    bad += st == 1;
+    nonfinite += st == 2;
   }
   if (nonfinite)
     throw Error(TNBP_ENOTCONV, std::to_string(nonfinite) + " edge(s) with non-finite messages at truncation");

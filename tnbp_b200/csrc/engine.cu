@@ -36,6 +36,7 @@
 #include "tc_gram.cuh"
 #include "tc_leg64.cuh"
 #include "tc_leg_gram.cuh"
+#include "tc_pair.cuh"
 #include "site_sweep.cuh"
 #include "trace.h"
 #include "truncate.cuh"
@@ -438,6 +439,8 @@ struct Unit {
   std::vector<PlanOp> ops;
   std::vector<int> targets;  // targets with a plain Gram (of result[t])
   std::vector<Fused> fused;  // targets with the fused absorption + Gram
+  int pair_src = -2;         // slot of W for the unit's pair of targets (k_pair_gram_tc); -2: none
+  int pair = 0;              // the targets are legs 2 pair and 2 pair + 1
   std::map<int, int> buf_of_slot;
   int nbuf = 0;
   int nlevels = 0;
@@ -485,6 +488,22 @@ Unit make_unit(int site, int u, const std::vector<PlanOp>& all, const SitePlanne
     U.nlevels = std::max(U.nlevels, op.level + 1);
   }
   U.nbuf = (int)busy_until.size();
+  return U;
+}
+
+// Unit u of a degree-4 site whose two targets (legs 2u, 2u + 1) go through
+// k_pair_gram_tc: only the absorption of the two other legs stays.
+Unit make_pair_unit(int site, int u, const std::vector<PlanOp>& all) {
+  Unit U;
+  U.site = site;
+  U.pair = u;
+  for (const auto& op : all)
+    if (op.site == site && op.unit == u && op.level < 2) {
+      U.buf_of_slot[op.dst] = op.level;
+      if (op.level == 1) U.pair_src = op.dst;
+      U.ops.push_back(op);
+    }
+  U.nbuf = U.nlevels = 2;
   return U;
 }
 }  // namespace
@@ -742,7 +761,9 @@ void Job::build_plan() {
       return reduced_sweeps(prec) && tcgen05_enabled() && leg_gram_enabled() && tc::leg_gram_ok(sh[t], sh[w]);
     };
     const int nunits = gs >= 2 ? 2 : 1;
-    for (int u = 0; u < nunits; ++u) units.push_back(make_unit(s, u, ops, sp, fuse));
+    const bool pair = reduced_sweeps(prec) && tcgen05_enabled() && !leg_gram_enabled() && tc::pair_ok(sh.data(), gs);
+    for (int u = 0; u < nunits; ++u)
+      units.push_back(pair ? make_pair_unit(s, u, ops) : make_unit(s, u, ops, sp, fuse));
   }
   // 2. waves of consecutive units within the byte budget (at least one unit)
   if (!tuning) choose_wave_budget();
@@ -822,6 +843,7 @@ void Job::build_plan() {
   std::vector<Pending> pend;      // one per target, in message order
   std::vector<size_t> gram_part;  // pend index of each plain Gram task
   std::vector<size_t> lg_part;    // pend index of each fused task
+  std::vector<size_t> pair_part;  // pend indices of each pair task's two targets
   for (size_t w = 0; w < waves.size(); ++w) {
     WaveHost& W = plan.waves[w];
     int nlev = 0;
@@ -873,6 +895,36 @@ void Job::build_plan() {
         part += (size_t)g1.nchunk * g1.C * g1.C;
         plan.gram.push_back(g1);
         plan.gram_blocks.push_back((long long)g1.nchunk * g1.ctiles * g1.ctiles);
+      }
+      if (U.pair_src >= -1) {
+        const int x = 2 * U.pair, y = x + 1;
+        LegPairTask pt{};
+        pt.W = slot_ptr(ui, U.pair_src);
+        pt.V = sweep_vptr(U.site);
+        pt.L1 = 1;
+        for (int k = 0; k < x; ++k) pt.L1 *= sh[k];
+        pt.Dx = sh[x];
+        pt.Dy = sh[y];
+        pt.n_outer = (long long)(site_elems(U.site) / ((size_t)sh[x] * sh[y]));
+        pt.planes = tc::pair_planes(pt.Dx, pt.Dy);
+        pt.div_l = make_fastdiv((uint32_t)pt.L1);
+        // about 16 chunks per pair, so that one site's pairs still fill 32
+        // CTAs; a chunk of up to 32 tiles hides its start and end
+        const long long tiles = (pt.n_outer + pt.planes - 1) / pt.planes;
+        pt.chunk_tiles = (int)std::max<long long>(1, std::min<long long>(32, (tiles + 15) / 16));
+        pt.nchunk = (int)((tiles + pt.chunk_tiles - 1) / pt.chunk_tiles);
+        W.pairs.push_back((int)plan.pair[0].size());
+        for (int t : {x, y}) {
+          W.msgs.push_back((int)pend.size());
+          pair_part.push_back(pend.size());
+          pend.push_back({U.site, t, part, pt.nchunk, sh[t]});
+          part += (size_t)pt.nchunk * sh[t] * sh[t];
+        }
+        for (int par = 0; par < 2; ++par) {
+          pt.Ex = mptr(par, g.in_msg(U.site, x));
+          pt.Ey = mptr(par, g.in_msg(U.site, y));
+          plan.pair[par].push_back(pt);
+        }
       }
       for (const auto& f : U.fused) {
         const int t = f.target, w2 = f.leg, p1 = std::min(t, w2), p2 = std::max(t, w2);
@@ -943,6 +995,11 @@ void Job::build_plan() {
   for (size_t i = 0; i < plan.gram.size(); ++i) plan.gram[i].partial = partial + pend[gram_part[i]].part_off;
   for (size_t i = 0; i < lg_part.size(); ++i)
     for (int par = 0; par < 2; ++par) plan.lg[par][i].partial = partial + pend[lg_part[i]].part_off;
+  for (size_t i = 0; i < plan.pair[0].size(); ++i)
+    for (int par = 0; par < 2; ++par) {
+      plan.pair[par][i].part_x = partial + pend[pair_part[2 * i]].part_off;
+      plan.pair[par][i].part_y = partial + pend[pair_part[2 * i + 1]].part_off;
+    }
   for (int par = 0; par < 2; ++par) plan.msg[par].clear();
   for (size_t i = 0; i < pend.size(); ++i) {
     const int mo = g.out_msg(pend[i].s, pend[i].t);
@@ -998,6 +1055,18 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
     L.nblocks = nblocks;
     L.max_din = max_din;
     b.launches.push_back(L);
+  };
+  auto add_pairs = [&](int kind, std::vector<LegPairTask>* pt, std::vector<long long>* pb, const long long* tiles) {
+    std::vector<LegPairTask> all(pt[0]);
+    std::vector<long long> beg(pb[0]);
+    all.insert(all.end(), pt[1].begin(), pt[1].end());
+    beg.insert(beg.end(), pb[1].begin(), pb[1].end());
+    if (all.empty()) return;
+    add(kind, all, beg, tiles[0], 0);
+    SweepLaunch& L = b.launches.back();
+    L.ntask = (int)pt[0].size();
+    L.ntask8 = (int)pt[1].size();
+    L.nblocks8 = tiles[1];
   };
   // The kernel is chosen per task, never per launch: complex64 tasks whose
   // tile is a contiguous byte range (tc::bulk_mode) run on the bulk-staged
@@ -1066,8 +1135,10 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
     std::vector<GramTask> gt, gt2, gt3;
     std::vector<long long> gb, gb2, gb3, lb;
     std::vector<LegGramTask> lt;
+    std::vector<LegPairTask> pt[2];  // 4 and 8 planes per tile
+    std::vector<long long> pb[2];
     std::vector<MsgTask> mt;
-    long long nb = 0, nb2 = 0, nb3 = 0, nlb = 0;
+    long long nb = 0, nb2 = 0, nb3 = 0, nlb = 0, npb[2] = {0, 0};
     for (auto& e : entries) {
       const auto& P = e.job->plan;
       if (w >= P.waves.size()) continue;
@@ -1077,6 +1148,14 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
         lb.push_back(nlb);
         nlb += l1.nchunk;
         lt.push_back(l1);
+      }
+      for (int pi : P.waves[w].pairs) {
+        LegPairTask p1 = P.pair[e.parity][pi];
+        const int k = p1.planes == 4 ? 0 : 1;
+        p1.block_begin = npb[k];
+        pb[k].push_back(npb[k]);
+        npb[k] += (p1.n_outer + p1.planes - 1) / p1.planes;
+        pt[k].push_back(p1);
       }
       for (int mi : P.waves[w].msgs) mt.push_back(P.msg[e.parity][mi]);
       for (int gi : P.waves[w].grams) {
@@ -1100,6 +1179,7 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
       }
     }
     add(SweepLaunch::LEG_GRAM, lt, lb, nlb, 0);
+    add_pairs(SweepLaunch::PAIR_GRAM, pt, pb, npb);
     add(SweepLaunch::GRAM_TC, gt2, gb2, nb2, 0);
     add(SweepLaunch::GRAM_T64, gt3, gb3, nb3, 0);
     add(SweepLaunch::GRAM_CORE, gt, gb, nb, 0);
@@ -1156,6 +1236,16 @@ void launch_gram_f64(const GramTask* tasks, const long long* begins, int ntask, 
 }
 long long leg_tiles_f64(long long L, long long R) { return dm::leg_tiles(L, R); }
 
+// CTAs of a pair launch for its two kinds of task: one CTA per SM (about 226
+// KB of shared memory each), shared out by their tiles.
+static std::pair<int, int> pair_grid(const SweepLaunch& L) {
+  const long long sms = num_sms(), all = L.nblocks + L.nblocks8;
+  if (!L.nblocks8) return {(int)std::min(sms, L.nblocks), 0};
+  if (!L.nblocks) return {0, (int)std::min(sms, L.nblocks8)};
+  const long long four = std::max<long long>(1, std::min(sms - 1, (sms * L.nblocks + all / 2) / all));
+  return {(int)std::min(four, L.nblocks), (int)std::min(sms - four, L.nblocks8)};
+}
+
 template <typename R, typename MR>
 static int launch_batch_t(const SweepBatch& b, cudaStream_t stream) {
   const char* base = static_cast<const char*>(b.arena.p);
@@ -1205,6 +1295,12 @@ static int launch_batch_t(const SweepBatch& b, cudaStream_t stream) {
         k_leg_gram_tc<MR><<<(unsigned)L.nblocks, 256, tc::leg_gram_smem_bytes(), stream>>>(
             static_cast<const LegGramTask*>(tasks), begins, L.ntask);
         break;
+      case SweepLaunch::PAIR_GRAM: {
+        const auto grid = pair_grid(L);
+        k_pair_gram_tc<MR><<<(unsigned)(grid.first + grid.second), tc::kPairThreads, tc::pair_smem_bytes(), stream>>>(
+            static_cast<const LegPairTask*>(tasks), begins, L.ntask, L.nblocks, L.ntask8, L.nblocks8, grid.first);
+        break;
+      }
       case SweepLaunch::GRAM_CORE:
         if constexpr (sizeof(R) == 8)
           launch_gram_f64(static_cast<const GramTask*>(tasks), begins, L.ntask, L.nblocks, stream);
@@ -1247,6 +1343,8 @@ static void tc_attr() {
                           (int)tc::leg64_smem_bytes()));
   CK(cudaFuncSetAttribute(k_leg_gram_tc<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)tc::leg_gram_smem_bytes()));
+  CK(cudaFuncSetAttribute(k_pair_gram_tc<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          (int)tc::pair_smem_bytes()));
   if (!attr_done(gram_flags)) {
     CK(cudaFuncSetAttribute(k_gram_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::gram_smem_bytes()));
     CK(cudaFuncSetAttribute(k_gram_tc64, cudaFuncAttributeMaxDynamicSharedMemorySize,

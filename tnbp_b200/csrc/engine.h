@@ -80,18 +80,21 @@ struct WaveHost {
   std::vector<LevelHost> levels;
   std::vector<int> grams;  // indices into SweepPlan::gram
   std::vector<int> lgs;    // indices into SweepPlan::lg
+  std::vector<int> pairs;  // indices into SweepPlan::pair
   std::vector<int> msgs;   // indices into SweepPlan::msg (one per target)
 };
 
 // One kernel launch of a sweep batch; its task arrays live in the batch's
 // arena at the given byte offsets.
 struct SweepLaunch {
-  enum Kind { LEG_BULK, LEG_T64, LEG_TC, LEG_CORE, GRAM_TC, GRAM_T64, GRAM_CORE, LEG_GRAM, MSG, SUM, SITE };
+  enum Kind { LEG_BULK, LEG_T64, LEG_TC, LEG_CORE, GRAM_TC, GRAM_T64, GRAM_CORE, LEG_GRAM, PAIR_GRAM, MSG, SUM, SITE };
   int kind;
   size_t tasks_off, begins_off;
   int ntask;
   long long nblocks;
   int max_din;
+  int ntask8 = 0;          // PAIR_*: tasks of eight planes per tile, after ntask of four
+  long long nblocks8 = 0;  // and their tiles
 };
 
 // Device task arrays of one sweep launch sequence; built from one job (the
@@ -120,6 +123,7 @@ struct SweepPlan {
   std::vector<GramTask> gram;
   std::vector<long long> gram_blocks;  // blocks of each gram task (CUDA-core kernel)
   std::vector<LegGramTask> lg[2];      // fused last absorption + Gram, per parity
+  std::vector<LegPairTask> pair[2];       // both messages of a pair of legs, per parity
   std::vector<MsgTask> msg[2];         // one per target, per message-arena parity
   std::vector<SiteTask> site[2];       // sites swept whole on chip (k_site_sweep), per parity
   SweepBatch single[2];

@@ -255,6 +255,22 @@ struct LegGramTask {
   long long block_begin; // exclusive prefix of nchunk over tasks
 };
 
+// Both messages of a pair of legs of a degree-4 site (tc_pair.cuh): the
+// plane's element (x, y) of outer index o = lo + L1 hi lies at
+// lo + L1 (x + Dx y) + L1 Dx Dy hi.
+struct LegPairTask {
+  const void* W;         // complex64, the other two bond legs absorbed
+  const void* V;         // complex64 site tensor
+  const void* Ex;        // Dx x Dx message absorbed on leg x (element type MR)
+  const void* Ey;        // Dy x Dy
+  double2* part_x;       // [nchunk][Dx * Dx]
+  double2* part_y;       // [nchunk][Dy * Dy]
+  long long L1, n_outer; // n_outer < 2^31
+  int Dx, Dy, planes, chunk_tiles, nchunk;
+  long long block_begin; // exclusive prefix of tiles over tasks
+  FastDiv div_l;         // by L1
+};
+
 // One small site's whole sweep (k_site_sweep, site_sweep.cuh).
 struct SiteTask {
   const void* V;               // site tensor (R), column-major (D_0, ..., D_{g-1}, d)

@@ -1,0 +1,589 @@
+// Both messages of a pair of legs on tcgen05 (sm_100a), for the complex64 and
+// mixed sweeps.  A site's legs are taken as a plane (x, y) and an outer index
+// o (every other leg and the physical one); with W the site tensor after the
+// two other bond legs' messages were absorbed and V the site tensor,
+//   N_x[x, x'] = sum_{o, y}  (sum_y2 W[x, y2, o] E_y[y2, y]) conj(V[x', y, o])
+//   N_y[y, y'] = sum_{o, x}  (sum_x2 W[x2, y, o] E_x[x2, x]) conj(V[x, y', o])
+// -- the last absorption of bp.h:137-152 for both targets and their Grams
+// (bp.h:157-166) -- in one pass over W and V: the absorbed tensors stay on
+// chip.  Degree-4 sites with every dim <= 32 (the others keep the separate
+// leg and Gram kernels).
+//
+// Why: level by level, these two absorptions and Grams read and write a site
+// tensor 12 times per pair; here 2 reads remain, and the bound moves from
+// HBM and launch tails to shared memory (operand stores and MMA reads, about
+// 6000 cycles per tile at D = 32) and the conversions.  MEASURED
+//
+// A tile is P planes (P Dx, P Dy <= 128 rows): raw complex64 planes arrive by
+// cp.async, two tiles in flight, element (o, x, y) at y PE + o Dx + x with PE
+// odd, so that rows (o, x) over y and rows (o, y) over x both read without
+// bank conflicts.  Per target (say x; for y the roles swap):
+//   1. rows (o, x) of W, split hi/lo (3xTF32), go to tensor memory as the A
+//      operand; D1 = A_re [E_re | E_im], D2 = A_im [E_re | E_im] (hi.hi +
+//      hi.lo + lo.hi, A from TMEM, 24 MMAs of N = 64 at D = 32), so only the
+//      two 64-column halves of E are kept in shared memory;
+//      P_re = D1_re - D2_im, P_im = D1_im + D2_re
+//   2. P and the matching rows of V become the Gram's operands, half of the y
+//      range at a time: rows [re_hi; im_hi; re_lo; im_lo] x 32 of up to 64
+//      contraction columns (o, y); one M = 128, N = 128 MMA per 8 columns
+//      gives all four hi/lo products
+//   3. the tile's FP32 Gram is added to FP64 registers.
+// A chunk of tiles ends in one FP64 partial per target, reduced by
+// k_msg_finalize in a fixed order.
+//
+// Every wait is bounded: on timeout the CTA records g_tc_error, waits once
+// more (bounded) for its MMAs, frees its TMEM and returns without writing
+// its partials.
+#pragma once
+#include <cstdint>
+#include <type_traits>
+
+#include "tc_gram.cuh"
+
+namespace tnbp {
+
+namespace tc {
+constexpr int kPairWarps = 16;                               // converting warps
+constexpr int kPairLoaders = 3;                              // loading warps, beside one that issues the MMAs
+constexpr int kPairThreads = 32 * (kPairWarps + 1 + kPairLoaders);
+// Registers per thread after the split: 512 x 112 + 128 x 32 = 640 x 96, what
+// the launch gives the CTA (64 of the 112 are the FP64 sums).
+constexpr int kPairRegsWork = 112, kPairRegsFeed = 32;
+static_assert(kPairWarps * kPairRegsWork + (1 + kPairLoaders) * kPairRegsFeed <= 96 * (kPairWarps + 1 + kPairLoaders),
+              "register split");
+constexpr int kPairRawElems = 32 * 129;                      // one tensor's planes of a tile
+constexpr int kPairWaitLimit = 1 << 22;
+constexpr uint32_t kPairE = 64 * 32 * 4;                     // one of E's operands (N = 64, K = 32)
+constexpr uint32_t kPairOp = 128 * 64 * 4;                   // one Gram operand of a stage (128 rows, 64 columns)
+__host__ __device__ constexpr size_t pair_smem_bytes() {
+  return 1024 + 4 * (size_t)kPairE + 2 * (size_t)kPairOp + 4 * (size_t)kPairRawElems * 8 + 128;
+}
+// Planes per tile: 4 (8 up to dimension 16), so that the padded rows of
+// either target stay within 128 and a Gram stage of 16 (8) of their columns
+// within 64.
+__host__ __device__ inline int pair_planes(int Dx, int Dy) { return (Dx > Dy ? Dx : Dy) <= 16 ? 8 : 4; }
+// Element x of plane o lies at x ^ pair_swizzle(o): loads that run along o
+// then write distinct banks; groups of four stay together.
+__host__ __device__ __forceinline__ uint32_t pair_swizzle(uint32_t o, uint32_t Xp) { return 4u * (o & (Xp % 16 == 0 ? 3u : 1u)); }
+
+// The sites that take it: degree 4, every bond dimension at most 32.
+__host__ __device__ inline bool pair_ok(const int* D, int g) {
+  return g == 4 && D[0] <= 32 && D[1] <= 32 && D[2] <= 32 && D[3] <= 32;
+}
+
+__device__ __forceinline__ void mma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+  const uint32_t z = 0;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}\n"
+      :
+      : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(z), "r"(z), "r"(z), "r"(z));
+}
+__device__ __forceinline__ void tmem_st4(uint32_t addr, float4 v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(__float_as_uint(v.x)),
+               "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w))
+               : "memory");
+}
+// Four columns of this warp's lanes; the caller waits (tmem_ld_wait) before
+// it uses them.
+__device__ __forceinline__ void tmem_ld4_async(uint32_t addr, float* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+               : "r"(addr));
+}
+// Waits for the loads; the values pass through it, so that no use of them can
+// be moved before it.
+__device__ __forceinline__ void tmem_ld_wait16(float* a, float* b, float* c, float* d) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+f"(a[0]), "+f"(a[1]), "+f"(a[2]), "+f"(a[3]), "+f"(b[0]), "+f"(b[1]), "+f"(b[2]), "+f"(b[3]),
+                 "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]), "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               :
+               : "memory");
+}
+
+// x = hi + lo with hi = x rounded to 11 significant bits (half away, as
+// cvt.rna.tf32 does) and lo = x - hi exact, of which the tensor core reads the
+// upper 11 bits: lo has at most 12 below its sign, so that is off by at most
+// one unit of x's last place, as far as rounding lo would be.  Three
+// instructions per value; the conversion instruction expands to four and
+// both roundings by it bound the kernel.  A NaN reaches the product in lo.
+__device__ __forceinline__ void split1(float x, float& h, float& l) {
+  h = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
+  l = x - h;
+}
+__device__ __forceinline__ void split4(float4 v, float4& h, float4& l) {
+  split1(v.x, h.x, l.x);
+  split1(v.y, h.y, l.y);
+  split1(v.z, h.z, l.z);
+  split1(v.w, h.w, l.w);
+}
+__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t phase) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(done)
+      : "r"(addr), "r"(phase)
+      : "memory");
+  return done != 0;
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t addr) {
+  asm volatile("{\n\t.reg .b64 s;\n\tmbarrier.arrive.shared::cta.b64 s, [%0];\n\t}\n" ::"r"(addr) : "memory");
+}
+// The chunks of one CTA: those whose first tile lies in [lo, hi) of all tasks'
+// tiles (begins: exclusive prefix of tiles), so CTAs get equal shares of
+// uneven tasks while a task's chunks depend on the task alone.
+struct PairChunks {
+  const LegPairTask* tasks;
+  const long long* begins;
+  int ntask, ti, chunk;
+  long long hi;
+  __device__ PairChunks(const LegPairTask* t, const long long* b, int n, long long lo, long long h)
+      : tasks(t), begins(b), ntask(n), ti(find_task(b, n, lo)), chunk(0), hi(h) {
+    chunk = (int)((lo - begins[ti] + tasks[ti].chunk_tiles - 1) / tasks[ti].chunk_tiles);
+  }
+  __device__ bool valid() {
+    while (ti < ntask && chunk >= tasks[ti].nchunk) {
+      ++ti;
+      chunk = 0;
+    }
+    return ti < ntask && begins[ti] + (long long)chunk * tasks[ti].chunk_tiles < hi;
+  }
+};
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void cp8(float2* dst, const float2* src, bool valid) {
+  const uint32_t d = smem_u32(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
+}
+}  // namespace tc
+
+// CTA `block` of `nblock`, all tasks of P planes per tile.
+template <typename MR, uint32_t P>
+__device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks, const long long* __restrict__ begins, int ntask,
+                                          long long ntile_all, uint32_t block, uint32_t nblock) {
+  using namespace tc;
+  extern __shared__ __align__(1024) unsigned char pr_smem_raw[];
+  unsigned char* smem = pr_smem_raw + ((1024 - (smem_u32(pr_smem_raw) & 1023)) & 1023);
+  unsigned char* e_op = smem;                       // E_y hi, lo, E_x hi, lo
+  unsigned char* g_op = e_op + 4 * kPairE;          // Gram operands of P and of V
+  float2* raw = reinterpret_cast<float2*>(g_op + 2 * kPairOp);  // [tile parity][W, V]
+  // mbarriers: leg operands ready, done; Gram operands ready, done; per tile
+  // parity: tile arrived, used
+  uint64_t* bars = reinterpret_cast<uint64_t*>(raw + 4 * kPairRawElems);
+  const uint32_t bar_leg = smem_u32(bars), bar_leg_done = bar_leg + 8, bar_ready = bar_leg + 16, bar_done = bar_leg + 24,
+                 bar_full = bar_leg + 32, bar_free = bar_leg + 48;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  volatile int* fail = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+
+  // persistent: an equal share of the tiles
+  const long long share = (ntile_all + nblock - 1) / nblock, first_tile = block * share;
+  const long long last_tile = min(ntile_all, first_tile + share);
+  if (first_tile >= last_tile) return;
+  // groups of four columns in a row; a Gram stage holds up to `per` of them,
+  // of every plane: one or two stages per target
+  constexpr uint32_t per = P == 4 ? 4u : 2u;
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t count = i == 1 || i == 3 ? 1u : i == 4 || i == 5 ? 32u * kPairLoaders : (uint32_t)kPairWarps;
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bars + i)), "r"(count));
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    *fail = 0;
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  constexpr uint32_t kColP = 128, kColN = 256;  // A operand at 0, D1 at 128, D2 at 192, N_x at 256, N_y at 384
+
+  // A bounded wait by a whole warp; false (for the whole warp) when it or
+  // any other thread of the CTA gave up.
+  auto wait = [&](uint32_t bar, uint32_t phase) -> bool {
+    bool ok = __all_sync(0xffffffffu, mbar_try(bar, phase));
+    for (int i = 0; i < kPairWaitLimit && !ok; ++i) {
+      ok = __all_sync(0xffffffffu, mbar_try(bar, phase));
+      if (!ok && (i & 1023) == 1023 && __any_sync(0xffffffffu, *fail)) break;
+    }
+    if (!ok) *fail = 1;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    return ok;
+  };
+
+  // The register split is made inside each role's branch, so that no path
+  // leads from the smaller share into the converting warps' code.
+  if (warp < kPairWarps) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPairRegsWork));
+    // this thread's row of a tile, (o, x) or (o, y); of its groups of four
+    // columns, j, warps 4 g .. 4 g + 3 hold those with j % 4 == g
+    const int row = 32 * (warp & 3) + lane;
+    const uint32_t g = (uint32_t)warp >> 2;
+    const uint32_t lanes = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    double acc[2][16];
+    // of the chunk's task: padded dimensions and groups, this thread's place
+    // in a tile and in the operands
+    uint32_t Xp = 0, Yp = 0, PE = 0, gx = 0, gy = 0, ox = 0, xx = 0, oy = 0, yy = 0, base_x = 0, base_y = 0, swz_y = 0, op_x = 0,
+             op_y = 0;
+
+    auto drain = [&](double (&a)[16], uint32_t col) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float v[8], u[8];
+        const uint32_t c = lanes + col + 16u * g + 8u * h;
+        tmem_ld4_async(c, v);
+        tmem_ld4_async(c + 4, v + 4);
+        tmem_ld4_async(c + 64, u);
+        tmem_ld4_async(c + 68, u + 4);
+        tmem_ld_wait16(v, v + 4, u, u + 4);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[8 * h + i] += (double)(v[i] + u[i]);
+      }
+    };
+    // group j (four columns) of this row: along y for (o, x), along x for (o, y)
+    auto read4 = [&](const float2* t, bool target_y, uint32_t j, float4& re, float4& im) {
+      const uint32_t step = target_y ? 1u : PE;
+      const float2* p = t + (target_y ? base_y + ((4 * j) ^ swz_y) : base_x + 4 * j * PE);
+      const float2 a = p[0], b = p[step], c = p[2 * step], d = p[3 * step];
+      re = make_float4(a.x, b.x, c.x, d.x);
+      im = make_float4(a.y, b.y, c.y, d.y);
+    };
+    // rows of W as the A operand in tensor memory: [re_hi | im_hi | re_lo |
+    // im_lo] of 32 columns each
+    auto put_a = [&](const float2* w, bool target_y) {
+      const uint32_t n = target_y ? gx : gy;
+#pragma unroll
+      for (uint32_t i = 0; i < 2; ++i) {
+        const uint32_t j = g + 4 * i;
+        if (j < n) {
+          float4 re, im, rh, rl, ih, il;
+          const uint32_t c = lanes + 4 * j;
+          read4(w, target_y, j, re, im);
+          split4(re, rh, rl);
+          split4(im, ih, il);
+          tmem_st4(c, rh);
+          tmem_st4(c + 32u, ih);
+          tmem_st4(c + 64u, rl);
+          tmem_st4(c + 96u, il);
+        }
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    };
+    // P of this row: groups g and g + 4
+    float4 pr[2], pi[2];
+    auto get_p = [&](uint32_t n) {
+      const uint32_t Np = 4 * n, c0 = lanes + kColP + 4 * g;
+#pragma unroll
+      for (uint32_t i = 0; i < 2; ++i)
+        if (g + 4 * i < n) {
+          float rr[4], ri[4], ir[4], ii[4];
+          const uint32_t c = c0 + 16 * i;
+          tmem_ld4_async(c, rr);            // A_re E_re
+          tmem_ld4_async(c + Np, ri);       // A_re E_im
+          tmem_ld4_async(c + 64, ir);       // A_im E_re
+          tmem_ld4_async(c + 64 + Np, ii);  // A_im E_im
+          tmem_ld_wait16(rr, ri, ir, ii);
+          pr[i] = make_float4(rr[0] - ii[0], rr[1] - ii[1], rr[2] - ii[2], rr[3] - ii[3]);
+          pi[i] = make_float4(ri[0] + ir[0], ri[1] + ir[1], ri[2] + ir[2], ri[3] + ir[3]);
+        }
+    };
+    // four consecutive contraction columns of one row (re and im) into an
+    // operand: rows f (re_hi), 32 + f, 64 + f, 96 + f
+    auto put_op = [&](unsigned char* p, float4 re, float4 im) {
+      float4 rh, rl, ih, il;
+      split4(re, rh, rl);
+      split4(im, ih, il);
+      *reinterpret_cast<float4*>(p) = rh;
+      *reinterpret_cast<float4*>(p + 32 * 16) = ih;
+      *reinterpret_cast<float4*>(p + 64 * 16) = rl;
+      *reinterpret_cast<float4*>(p + 96 * 16) = il;
+    };
+    // operands written by this warp are visible to the MMAs issued after it
+    auto publish = [&](uint32_t bar) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    uint32_t gram_ph = 0, leg_ph = 0;  // parities of the MMAs waited for
+    auto gram_done = [&]() {
+      const bool r = wait(bar_done, gram_ph);
+      gram_ph ^= 1u;
+      return r;
+    };
+    auto leg_done = [&]() {
+      const bool r = wait(bar_leg_done, leg_ph);
+      leg_ph ^= 1u;
+      return r;
+    };
+    // One Gram stage: groups per s .. of every row.  A group's P is written by
+    // the warps that hold it, its V by those of (j + 2) % 4 == g (with two
+    // groups per stage the other ones), after the operands' last MMAs
+    // (`fresh`: there are none).
+    auto stage = [&](const float2* v, bool target_y, uint32_t n, uint32_t s, const float4& re, const float4& im, bool fresh) -> bool {
+      const uint32_t first = per * s, count = min(per, n - first);
+      const uint32_t jp = per == 4 ? g : g - first, jv = per == 4 ? (g + 2) & 3u : ((g + 2) & 3u) - first;  // within the stage
+      if (!fresh && !gram_done()) return false;
+      if ((target_y ? oy : ox) < P) {
+        unsigned char* op = g_op + (target_y ? op_y : op_x);
+        if (jv < count) {
+          float4 vr, vi;
+          read4(v, target_y, first + jv, vr, vi);
+          put_op(op + kPairOp + jv * (P * 128 * 16), vr, vi);
+        }
+        if (jp < count) put_op(op + jp * (P * 128 * 16), re, im);
+      }
+      publish(bar_ready);
+      return true;
+    };
+
+    auto tile_ready = [&](uint32_t i) { return wait(bar_full + 8u * (i & 1u), (i >> 1) & 1u); };
+    bool ok = true;
+    uint32_t T = 0;  // tiles so far: tile T arrives in raw[T & 1]
+    int cur = -1;
+    for (PairChunks ch(tasks, begins, ntask, first_tile, last_tile); ok && ch.valid(); ++ch.chunk) {
+    const LegPairTask& tk = tasks[ch.ti];
+    const int ntile = min(tk.chunk_tiles, (int)((tk.n_outer + P - 1) / P) - ch.chunk * tk.chunk_tiles);
+    if (ch.ti != cur) {  // no MMA is in flight between chunks
+      cur = ch.ti;
+      Xp = uniform(((uint32_t)tk.Dx + 7u) & ~7u);
+      Yp = uniform(((uint32_t)tk.Dy + 7u) & ~7u);
+      PE = (P * Xp) | 1u;
+      gx = Xp / 4;
+      gy = Yp / 4;
+      ox = (uint32_t)row / Xp;
+      xx = (uint32_t)row - ox * Xp;
+      oy = (uint32_t)row / Yp;
+      yy = (uint32_t)row - oy * Yp;
+      base_x = ox < P ? ox * Xp + (xx ^ pair_swizzle(ox, Xp)) : 0;  // + y PE
+      base_y = oy < P ? yy * PE + oy * Xp : 0;                      // + (x ^ swz_y)
+      swz_y = pair_swizzle(oy, Xp);
+      op_x = ox * (128 * 16) + (xx >> 3) * 128 + (xx & 7) * 16;  // + P 2048 per group
+      op_y = oy * (128 * 16) + (yy >> 3) * 128 + (yy & 7) * 16;
+      // E operands: element (n, k) of N = 2 Np rows (re, im), K = Np columns
+      for (int leg = 0; leg < 2; ++leg) {
+        const int D = leg == 0 ? tk.Dy : tk.Dx, Np = leg == 0 ? (int)Yp : (int)Xp, N2 = 2 * Np;
+        const typename cvec<MR>::type* E = static_cast<const typename cvec<MR>::type*>(leg == 0 ? tk.Ey : tk.Ex);
+        unsigned char* hi_op = e_op + (size_t)leg * 2 * kPairE;
+        if (lane < Np) {
+          for (int n = warp; n < N2; n += kPairWarps) {
+            const int c = n < Np ? n : n - Np;
+            double v = 0.0;
+            if (lane < D && c < D) {
+              const double2 m = to_d2(E[lane + (long long)D * c]);
+              v = n < Np ? m.x : m.y;
+            }
+            // the remainder in FP64, so that complex128 messages keep their low bits
+            const float h = to_tf32((float)v), l = to_tf32((float)(v - (double)h));
+            *reinterpret_cast<float*>(hi_op + kmajor_off(n, lane, N2)) = h;
+            *reinterpret_cast<float*>(hi_op + kPairE + kmajor_off(n, lane, N2)) = l;
+          }
+        }
+        __syncwarp();
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) acc[0][i] = acc[1][i] = 0.0;
+    if ((ok = tile_ready(T))) {
+      put_a(raw + (size_t)(T & 1u) * 2 * kPairRawElems, false);
+      publish(bar_leg);
+    }
+    for (int t = 0; t < ntile && ok; ++t, ++T) {
+      const float2* wr = raw + (size_t)(T & 1u) * 2 * kPairRawElems;
+      const float2* vr = wr + kPairRawElems;
+      // what overlaps the MMAs of each stage is the work that follows it
+      if (!(ok = leg_done())) break;
+      get_p(gy);
+      if (!(ok = stage(vr, false, gy, 0, pr[0], pi[0], t == 0))) break;
+      put_a(wr, true);
+      publish(bar_leg);
+      if (gy > per && !(ok = stage(vr, false, gy, 1, pr[per / 4], pi[per / 4], false))) break;
+      if (t > 0) drain(acc[1], kColN + 128u);  // the last tile's Gram of y
+      if (!(ok = leg_done())) break;
+      get_p(gx);
+      if (!(ok = stage(vr, true, gx, 0, pr[0], pi[0], false))) break;
+      if (t + 1 < ntile) {
+        if (!(ok = tile_ready(T + 1))) break;
+        put_a(raw + (size_t)((T + 1) & 1u) * 2 * kPairRawElems, false);
+        publish(bar_leg);
+      }
+      drain(acc[0], kColN);
+      if (gx > per && !(ok = stage(vr, true, gx, 1, pr[per / 4], pi[per / 4], false))) break;
+      if (lane == 0) mbar_arrive(bar_free + 8u * (T & 1u));
+    }
+    if (!ok || !(ok = gram_done())) break;
+    drain(acc[1], kColN + 128u);
+    // rows r and 64 + r of D, then N, through shared memory (the Gram
+    // operands are free)
+    double* dsum = reinterpret_cast<double*>(g_op);  // 64 x 64
+#pragma unroll
+    for (int target = 0; target < 2; ++target) {
+      const int C = target == 0 ? tk.Dx : tk.Dy;
+      double2* part = (target == 0 ? tk.part_x : tk.part_y) + (long long)ch.chunk * C * C;
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kPairWarps) : "memory");
+      if (row >= 64) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) dsum[(row - 64) + 65 * (16 * (int)g + i)] = acc[target][i];
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kPairWarps) : "memory");
+      if (row < 64) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) dsum[row + 65 * (16 * (int)g + i)] += acc[target][i];
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kPairWarps) : "memory");
+      if (lane < C)
+        for (int c2 = warp; c2 < C; c2 += kPairWarps) {
+          const double re = dsum[lane + 65 * c2] + dsum[32 + lane + 65 * (32 + c2)];
+          const double im = dsum[32 + lane + 65 * c2] - dsum[lane + 65 * (32 + c2)];
+          part[lane + (long long)C * c2] = make_double2(re, im);
+        }
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kPairWarps) : "memory");
+    }  // chunks
+    if (!ok && tid == 0) {
+      // MMAs in flight get one more bounded wait before TMEM is freed
+      atomicExch(&g_tc_error, 1);
+      mbar_wait(bar_leg_done, 0u);
+      mbar_wait(bar_leg_done, 1u);
+      mbar_wait(bar_done, 0u);
+      mbar_wait(bar_done, 1u);
+    }
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairRegsFeed));
+    if (warp == kPairWarps) {
+      // ---- the issuing warp: MMAs in the order in which the others publish
+      // One elected thread issues; every value that goes into an MMA is made
+      // warp-uniform first and the loops are unrolled, so that operands sit
+      // in uniform registers (left to per-thread registers each MMA took 170
+      // cycles to issue, three times its own time).
+      const uint32_t base = uniform(tmem), up = P, uper = per;
+      const uint32_t e0 = uniform(smem_u32(e_op)), g0 = uniform(smem_u32(g_op));
+      uint32_t gram_ph = 0, leg_ph = 0, nx = 0, ny = 0;
+      bool ok = true;
+      auto leg = [&](uint32_t which) {  // 0: E_y (K = Yp), 1: E_x
+        ok = wait(bar_leg, leg_ph);
+        leg_ph ^= 1u;
+        if (!ok) return;
+        const uint32_t k8 = (which ? nx : ny) / 2, N2 = 16 * k8, idesc = idesc_tf32(128, 0) | ((N2 >> 3) << 17);
+        const uint64_t dh0 = smem_desc(e0 + which * 2 * kPairE, N2 * 16, 128), dl0 = smem_desc(e0 + which * 2 * kPairE + kPairE, N2 * 16, 128);
+        if (elect_one()) {
+#pragma unroll
+          for (uint32_t part = 0; part < 2; ++part)
+#pragma unroll
+            for (uint32_t s = 0; s < 4; ++s)
+              if (s < k8) {
+                const uint32_t d = base + kColP + 64u * part, ah = base + 32u * part + 8u * s;
+                const uint64_t dh = dh0 + s * 2 * N2, dl = dl0 + s * 2 * N2;  // two 16-byte K groups of N2 rows
+                mma_tf32_ts(d, ah, dh, idesc, s);
+                mma_tf32_ts(d, ah, dl, idesc, 1u);
+                mma_tf32_ts(d, ah + 64u, dh, idesc, 1u);
+              }
+          mma_commit(bar_leg_done);
+        }
+        __syncwarp();
+      };
+      const uint64_t da = smem_desc(g0, 128 * 16, 128), db = smem_desc(g0 + kPairOp, 128 * 16, 128);
+      auto stage = [&](uint32_t target, uint32_t count, uint32_t accumulate) {
+        ok = wait(bar_ready, gram_ph);
+        gram_ph ^= 1u;
+        if (!ok) return;
+        const uint32_t idesc = idesc_tf32(128, 128), d = base + kColN + 128u * target, ks = up * count / 2;
+        if (elect_one()) {
+#pragma unroll
+          for (uint32_t s = 0; s < 8; ++s)
+            if (s < ks) mma_tf32(d, da + 256 * s, db + 256 * s, idesc, accumulate + s);
+          mma_commit(bar_done);
+        }
+        __syncwarp();
+      };
+      for (PairChunks ch(tasks, begins, ntask, first_tile, last_tile); ok && ch.valid(); ++ch.chunk) {
+        const LegPairTask& tk = tasks[ch.ti];
+        const int ntile = min(tk.chunk_tiles, (int)((tk.n_outer + P - 1) / P) - ch.chunk * tk.chunk_tiles);
+        nx = uniform(2u * (((uint32_t)tk.Dx + 7u) >> 3));
+        ny = uniform(2u * (((uint32_t)tk.Dy + 7u) >> 3));
+        leg(0);
+        for (int t = 0; t < ntile && ok; ++t) {
+          stage(0, min(uper, ny), 0u);
+          if (ok) leg(1);
+          if (ok && ny > uper) stage(0, ny - uper, 1u);
+          if (ok) stage(1, min(uper, nx), 0u);
+          if (ok && t + 1 < ntile) leg(0);
+          if (ok && nx > uper) stage(1, nx - uper, 1u);
+        }
+      }
+    } else {
+      // ---- the loading warps: for each y the P Xp elements (o, x) of a row,
+      // 32 at a time, in the order in which memory runs (x when the plane is
+      // contiguous, o when consecutive o are); padding is written as zeros
+      uint32_t T = 0;
+      bool ok = true;
+      const uint32_t y0 = (uint32_t)(warp - kPairWarps - 1);
+      for (PairChunks ch(tasks, begins, ntask, first_tile, last_tile); ok && ch.valid(); ++ch.chunk) {
+        const LegPairTask& tk = tasks[ch.ti];
+        const int ntile = min(tk.chunk_tiles, (int)((tk.n_outer + P - 1) / P) - ch.chunk * tk.chunk_tiles);
+        const uint32_t Dx = (uint32_t)tk.Dx, Dy = (uint32_t)tk.Dy, L1 = (uint32_t)tk.L1, O = (uint32_t)tk.n_outer;
+        const uint32_t Xp = (Dx + 7u) & ~7u, Yp = (Dy + 7u) & ~7u, PE = (P * Xp) | 1u;
+        const float2* __restrict__ Wg = static_cast<const float2*>(tk.W);
+        const ptrdiff_t VmW = static_cast<const float2*>(tk.V) - Wg;
+        for (int t = 0; t < ntile && ok; ++t, ++T) {
+          const uint32_t st = T & 1u;
+          if (T >= 2 && !(ok = wait(bar_free + 8u * st, ((T >> 1) - 1) & 1u))) break;
+          float2* dst = raw + (size_t)st * 2 * kPairRawElems;
+          const uint32_t o0 = (uint32_t)(ch.chunk * tk.chunk_tiles + t) * P;
+#pragma unroll 1
+          for (uint32_t el = (uint32_t)lane; el < P * Xp; el += 32) {
+            const uint32_t o = L1 == 1 ? el / Xp : el % P, x = L1 == 1 ? el - o * Xp : el / P;
+            const uint32_t oo = o0 + o, hi = fast_div(oo, tk.div_l), lo = oo - hi * L1;
+            const bool ok_ox = oo < O && x < Dx;
+            const float2* w = Wg + (ok_ox ? (size_t)lo + (size_t)L1 * (x + Dx * (y0 + Dy * (size_t)hi)) : 0);
+            const size_t dy = ok_ox ? (size_t)kPairLoaders * L1 * Dx : 0;
+            float2* d = dst + y0 * PE + o * Xp + (x ^ pair_swizzle(o, Xp));
+#pragma unroll 2
+            for (uint32_t y = y0; y < Yp; y += kPairLoaders) {
+              const bool in = ok_ox && y < Dy;
+              cp8(d, in ? w : Wg, in);
+              cp8(d + kPairRawElems, in ? w + VmW : Wg, in);
+              w += dy;
+              d += kPairLoaders * PE;
+            }
+          }
+          // this thread's arrival, when its copies have landed
+          asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar_full + 8u * st) : "memory");
+        }
+      }
+      asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+  }
+}
+
+// n4 tasks of four planes per tile (tiles4 tiles) on the first blocks4 CTAs,
+// then n8 of eight: one launch, so that neither kind waits for the other's
+// last CTAs.
+template <typename MR>
+__global__ void __launch_bounds__(tc::kPairThreads, 1)
+    k_pair_gram_tc(const LegPairTask* __restrict__ tasks, const long long* __restrict__ begins, int n4, long long tiles4, int n8,
+                   long long tiles8, int blocks4) {
+  if ((int)blockIdx.x < blocks4) pair_gram<MR, 4>(tasks, begins, n4, tiles4, blockIdx.x, (uint32_t)blocks4);
+  else pair_gram<MR, 8>(tasks + n4, begins + n4, n8, tiles8, blockIdx.x - (uint32_t)blocks4, gridDim.x - (uint32_t)blocks4);
+}
+
+}  // namespace tnbp

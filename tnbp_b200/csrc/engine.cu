@@ -492,18 +492,15 @@ Unit make_unit(int site, int u, const std::vector<PlanOp>& all, const SitePlanne
 }
 
 // Unit u of a degree-4 site whose two targets (legs 2u, 2u + 1) go through
-// k_pair_gram_tc: only the absorption of the two other legs stays.
-Unit make_pair_unit(int site, int u, const std::vector<PlanOp>& all) {
+// k_pair_gram_tc, after k_pair_absorb_tc has absorbed the other two legs into
+// the unit's one slot.
+Unit make_pair_unit(int site, int u) {
   Unit U;
   U.site = site;
   U.pair = u;
-  for (const auto& op : all)
-    if (op.site == site && op.unit == u && op.level < 2) {
-      U.buf_of_slot[op.dst] = op.level;
-      if (op.level == 1) U.pair_src = op.dst;
-      U.ops.push_back(op);
-    }
-  U.nbuf = U.nlevels = 2;
+  U.pair_src = 0;
+  U.buf_of_slot[0] = 0;
+  U.nbuf = 1;
   return U;
 }
 }  // namespace
@@ -763,7 +760,7 @@ void Job::build_plan() {
     const int nunits = gs >= 2 ? 2 : 1;
     const bool pair = reduced_sweeps(prec) && tcgen05_enabled() && !leg_gram_enabled() && tc::pair_ok(sh.data(), gs);
     for (int u = 0; u < nunits; ++u)
-      units.push_back(pair ? make_pair_unit(s, u, ops) : make_unit(s, u, ops, sp, fuse));
+      units.push_back(pair ? make_pair_unit(s, u) : make_unit(s, u, ops, sp, fuse));
   }
   // 2. waves of consecutive units within the byte budget (at least one unit)
   if (!tuning) choose_wave_budget();
@@ -896,25 +893,30 @@ void Job::build_plan() {
         plan.gram.push_back(g1);
         plan.gram_blocks.push_back((long long)g1.nchunk * g1.ctiles * g1.ctiles);
       }
-      if (U.pair_src >= -1) {
-        const int x = 2 * U.pair, y = x + 1;
-        LegPairTask pt{};
-        pt.W = slot_ptr(ui, U.pair_src);
-        pt.V = sweep_vptr(U.site);
-        pt.L1 = 1;
-        for (int k = 0; k < x; ++k) pt.L1 *= sh[k];
-        pt.Dx = sh[x];
-        pt.Dy = sh[y];
-        pt.n_outer = (long long)(site_elems(U.site) / ((size_t)sh[x] * sh[y]));
-        pt.planes = tc::pair_planes(pt.Dx, pt.Dy);
-        pt.div_l = make_fastdiv((uint32_t)pt.L1);
-        // about 16 chunks per pair, so that one site's pairs still fill 32
-        // CTAs; a chunk of up to 32 tiles hides its start and end
-        const long long tiles = (pt.n_outer + pt.planes - 1) / pt.planes;
-        pt.chunk_tiles = (int)std::max<long long>(1, std::min<long long>(32, (tiles + 15) / 16));
-        pt.nchunk = (int)((tiles + pt.chunk_tiles - 1) / pt.chunk_tiles);
+      if (U.pair_src >= 0) {
+        // legs x, x + 1 as a plane of site U.site
+        const auto pair_task = [&](int x) {
+          LegPairTask t{};
+          t.V = sweep_vptr(U.site);
+          t.W = slot_ptr(ui, U.pair_src);
+          t.L1 = 1;
+          for (int k = 0; k < x; ++k) t.L1 *= sh[k];
+          t.Dx = sh[x];
+          t.Dy = sh[x + 1];
+          t.n_outer = (long long)(site_elems(U.site) / ((size_t)sh[x] * sh[x + 1]));
+          t.planes = tc::pair_planes(t.Dx, t.Dy);
+          t.div_l = make_fastdiv((uint32_t)t.L1);
+          // about 16 chunks per pair, so that one site's pairs still fill 32
+          // CTAs; a chunk of up to 32 tiles hides its start and end
+          const long long tiles = (t.n_outer + t.planes - 1) / t.planes;
+          t.chunk_tiles = (int)std::max<long long>(1, std::min<long long>(32, (tiles + 15) / 16));
+          t.nchunk = (int)((tiles + t.chunk_tiles - 1) / t.chunk_tiles);
+          return t;
+        };
+        const int x = 2 * U.pair, other = 2 - x;
+        LegPairTask pt = pair_task(x), pa = pair_task(other);
         W.pairs.push_back((int)plan.pair[0].size());
-        for (int t : {x, y}) {
+        for (int t : {x, x + 1}) {
           W.msgs.push_back((int)pend.size());
           pair_part.push_back(pend.size());
           pend.push_back({U.site, t, part, pt.nchunk, sh[t]});
@@ -922,8 +924,11 @@ void Job::build_plan() {
         }
         for (int par = 0; par < 2; ++par) {
           pt.Ex = mptr(par, g.in_msg(U.site, x));
-          pt.Ey = mptr(par, g.in_msg(U.site, y));
+          pt.Ey = mptr(par, g.in_msg(U.site, x + 1));
+          pa.Ex = mptr(par, g.in_msg(U.site, other));
+          pa.Ey = mptr(par, g.in_msg(U.site, other + 1));
           plan.pair[par].push_back(pt);
+          plan.pabs[par].push_back(pa);
         }
       }
       for (const auto& f : U.fused) {
@@ -1068,6 +1073,13 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
     L.ntask8 = (int)pt[1].size();
     L.nblocks8 = tiles[1];
   };
+  auto push_pair = [](std::vector<LegPairTask>* pt, std::vector<long long>* pb, long long* tiles, LegPairTask t) {
+    const int k = t.planes == 4 ? 0 : 1;
+    t.block_begin = tiles[k];
+    pb[k].push_back(tiles[k]);
+    tiles[k] += (t.n_outer + t.planes - 1) / t.planes;
+    pt[k].push_back(t);
+  };
   // The kernel is chosen per task, never per launch: complex64 tasks whose
   // tile is a contiguous byte range (tc::bulk_mode) run on the bulk-staged
   // tcgen05 kernel, other tasks with Din, Dout <= 32 on the register-staged
@@ -1088,6 +1100,15 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
     add(SweepLaunch::SITE, sts, {}, (long long)sts.size(), (int)smem);
   }
   for (size_t w = 0; w < nw; ++w) {
+    {
+      std::vector<LegPairTask> pt[2];  // 4 and 8 planes per tile
+      std::vector<long long> pb[2];
+      long long tiles[2] = {0, 0};
+      for (auto& e : entries)
+        if (w < e.job->plan.waves.size())
+          for (int pi : e.job->plan.waves[w].pairs) push_pair(pt, pb, tiles, e.job->plan.pabs[e.parity][pi]);
+      add_pairs(SweepLaunch::PAIR_ABSORB, pt, pb, tiles);
+    }
     size_t nlev = 0;
     for (auto& e : entries)
       if (w < e.job->plan.waves.size()) nlev = std::max(nlev, e.job->plan.waves[w].levels.size());
@@ -1150,12 +1171,7 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
         lt.push_back(l1);
       }
       for (int pi : P.waves[w].pairs) {
-        LegPairTask p1 = P.pair[e.parity][pi];
-        const int k = p1.planes == 4 ? 0 : 1;
-        p1.block_begin = npb[k];
-        pb[k].push_back(npb[k]);
-        npb[k] += (p1.n_outer + p1.planes - 1) / p1.planes;
-        pt[k].push_back(p1);
+        push_pair(pt, pb, npb, P.pair[e.parity][pi]);
       }
       for (int mi : P.waves[w].msgs) mt.push_back(P.msg[e.parity][mi]);
       for (int gi : P.waves[w].grams) {
@@ -1236,14 +1252,14 @@ void launch_gram_f64(const GramTask* tasks, const long long* begins, int ntask, 
 }
 long long leg_tiles_f64(long long L, long long R) { return dm::leg_tiles(L, R); }
 
-// CTAs of a pair launch for its two kinds of task: one CTA per SM (about 226
-// KB of shared memory each), shared out by their tiles.
-static std::pair<int, int> pair_grid(const SweepLaunch& L) {
-  const long long sms = num_sms(), all = L.nblocks + L.nblocks8;
-  if (!L.nblocks8) return {(int)std::min(sms, L.nblocks), 0};
-  if (!L.nblocks) return {0, (int)std::min(sms, L.nblocks8)};
-  const long long four = std::max<long long>(1, std::min(sms - 1, (sms * L.nblocks + all / 2) / all));
-  return {(int)std::min(four, L.nblocks), (int)std::min(sms - four, L.nblocks8)};
+// CTAs of a persistent pair launch for its two kinds of task, `per_sm` CTAs
+// per SM shared out by their tiles.
+static std::pair<int, int> pair_grid(const SweepLaunch& L, int per_sm) {
+  const long long n = (long long)per_sm * num_sms(), all = L.nblocks + L.nblocks8;
+  if (!L.nblocks8) return {(int)std::min(n, L.nblocks), 0};
+  if (!L.nblocks) return {0, (int)std::min(n, L.nblocks8)};
+  const long long four = std::max<long long>(1, std::min(n - 1, (n * L.nblocks + all / 2) / all));
+  return {(int)std::min(four, L.nblocks), (int)std::min(n - four, L.nblocks8)};
 }
 
 template <typename R, typename MR>
@@ -1295,8 +1311,14 @@ static int launch_batch_t(const SweepBatch& b, cudaStream_t stream) {
         k_leg_gram_tc<MR><<<(unsigned)L.nblocks, 256, tc::leg_gram_smem_bytes(), stream>>>(
             static_cast<const LegGramTask*>(tasks), begins, L.ntask);
         break;
+      case SweepLaunch::PAIR_ABSORB: {
+        const auto grid = pair_grid(L, 2);
+        k_pair_absorb_tc<MR><<<(unsigned)(grid.first + grid.second), tc::kAbsorbThreads, tc::absorb_smem_bytes(), stream>>>(
+            static_cast<const LegPairTask*>(tasks), begins, L.ntask, L.nblocks, L.ntask8, L.nblocks8, grid.first);
+        break;
+      }
       case SweepLaunch::PAIR_GRAM: {
-        const auto grid = pair_grid(L);
+        const auto grid = pair_grid(L, 1);
         k_pair_gram_tc<MR><<<(unsigned)(grid.first + grid.second), tc::kPairThreads, tc::pair_smem_bytes(), stream>>>(
             static_cast<const LegPairTask*>(tasks), begins, L.ntask, L.nblocks, L.ntask8, L.nblocks8, grid.first);
         break;
@@ -1345,6 +1367,8 @@ static void tc_attr() {
                           (int)tc::leg_gram_smem_bytes()));
   CK(cudaFuncSetAttribute(k_pair_gram_tc<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)tc::pair_smem_bytes()));
+  CK(cudaFuncSetAttribute(k_pair_absorb_tc<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          (int)tc::absorb_smem_bytes()));
   if (!attr_done(gram_flags)) {
     CK(cudaFuncSetAttribute(k_gram_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::gram_smem_bytes()));
     CK(cudaFuncSetAttribute(k_gram_tc64, cudaFuncAttributeMaxDynamicSharedMemorySize,

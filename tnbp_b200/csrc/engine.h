@@ -87,7 +87,7 @@ struct WaveHost {
 // One kernel launch of a sweep batch; its task arrays live in the batch's
 // arena at the given byte offsets.
 struct SweepLaunch {
-  enum Kind { LEG_BULK, LEG_T64, LEG_TC, LEG_CORE, GRAM_TC, GRAM_T64, GRAM_CORE, LEG_GRAM, PAIR_GRAM, MSG, SUM, SITE };
+  enum Kind { LEG_BULK, LEG_T64, LEG_TC, LEG_CORE, GRAM_TC, GRAM_T64, GRAM_CORE, LEG_GRAM, PAIR_ABSORB, PAIR_GRAM, MSG, SUM, SITE };
   int kind;
   size_t tasks_off, begins_off;
   int ntask;
@@ -123,7 +123,8 @@ struct SweepPlan {
   std::vector<GramTask> gram;
   std::vector<long long> gram_blocks;  // blocks of each gram task (CUDA-core kernel)
   std::vector<LegGramTask> lg[2];      // fused last absorption + Gram, per parity
-  std::vector<LegPairTask> pair[2];       // both messages of a pair of legs, per parity
+  std::vector<LegPairTask> pair[2];    // both messages of a pair of legs, per parity
+  std::vector<LegPairTask> pabs[2];    // the absorption of the other pair before each
   std::vector<MsgTask> msg[2];         // one per target, per message-arena parity
   std::vector<SiteTask> site[2];       // sites swept whole on chip (k_site_sweep), per parity
   SweepBatch single[2];

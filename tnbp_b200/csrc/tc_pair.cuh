@@ -12,7 +12,10 @@
 // Why: level by level, these two absorptions and Grams read and write a site
 // tensor 12 times per pair; here 2 reads remain, and the bound moves from
 // HBM and launch tails to shared memory (operand stores and MMA reads, about
-// 6000 cycles per tile at D = 32) and the conversions.  MEASURED
+// 6000 cycles per tile at D = 32) and the conversions between hand-overs
+// (12600 to 15100 cycles per tile measured).  One 8x8 sweep at D = 32 (36
+// degree-4 sites): 3.96 ms in the separate kernels, 1.92 ms here; 6x6 at
+// D = 16: 0.17 -> 0.10 ms.
 //
 // A tile is P planes (P Dx, P Dy <= 128 rows): raw complex64 planes arrive by
 // cp.async, two tiles in flight, element (o, x, y) at y PE + o Dx + x with PE
@@ -165,6 +168,34 @@ __device__ __forceinline__ void cp8(float2* dst, const float2* src, bool valid) 
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
 }
 }  // namespace tc
+
+// The messages' operands, E_y then E_x, hi then lo each: element (n, k) of
+// N = 2 Np rows (re, im), K = Np columns; by `nwarp` warps.
+template <typename MR>
+__device__ __forceinline__ void build_pair_e(const LegPairTask& tk, unsigned char* e_op, uint32_t Xp, uint32_t Yp, int warp, int lane,
+                                             int nwarp) {
+  using namespace tc;
+  for (int leg = 0; leg < 2; ++leg) {
+    const int D = leg == 0 ? tk.Dy : tk.Dx, Np = leg == 0 ? (int)Yp : (int)Xp, N2 = 2 * Np;
+    const typename cvec<MR>::type* E = static_cast<const typename cvec<MR>::type*>(leg == 0 ? tk.Ey : tk.Ex);
+    unsigned char* hi_op = e_op + (size_t)leg * 2 * kPairE;
+    if (lane < Np) {
+      for (int n = warp; n < N2; n += nwarp) {
+        const int c = n < Np ? n : n - Np;
+        double v = 0.0;
+        if (lane < D && c < D) {
+          const double2 m = to_d2(E[lane + (long long)D * c]);
+          v = n < Np ? m.x : m.y;
+        }
+        // the remainder in FP64, so that complex128 messages keep their low bits
+        const float h = to_tf32((float)v), l = to_tf32((float)(v - (double)h));
+        *reinterpret_cast<float*>(hi_op + kmajor_off(n, lane, N2)) = h;
+        *reinterpret_cast<float*>(hi_op + kPairE + kmajor_off(n, lane, N2)) = l;
+      }
+    }
+    __syncwarp();
+  }
+}
 
 // CTA `block` of `nblock`, all tasks of P planes per tile.
 template <typename MR, uint32_t P>
@@ -374,27 +405,7 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
       swz_y = pair_swizzle(oy, Xp);
       op_x = ox * (128 * 16) + (xx >> 3) * 128 + (xx & 7) * 16;  // + P 2048 per group
       op_y = oy * (128 * 16) + (yy >> 3) * 128 + (yy & 7) * 16;
-      // E operands: element (n, k) of N = 2 Np rows (re, im), K = Np columns
-      for (int leg = 0; leg < 2; ++leg) {
-        const int D = leg == 0 ? tk.Dy : tk.Dx, Np = leg == 0 ? (int)Yp : (int)Xp, N2 = 2 * Np;
-        const typename cvec<MR>::type* E = static_cast<const typename cvec<MR>::type*>(leg == 0 ? tk.Ey : tk.Ex);
-        unsigned char* hi_op = e_op + (size_t)leg * 2 * kPairE;
-        if (lane < Np) {
-          for (int n = warp; n < N2; n += kPairWarps) {
-            const int c = n < Np ? n : n - Np;
-            double v = 0.0;
-            if (lane < D && c < D) {
-              const double2 m = to_d2(E[lane + (long long)D * c]);
-              v = n < Np ? m.x : m.y;
-            }
-            // the remainder in FP64, so that complex128 messages keep their low bits
-            const float h = to_tf32((float)v), l = to_tf32((float)(v - (double)h));
-            *reinterpret_cast<float*>(hi_op + kmajor_off(n, lane, N2)) = h;
-            *reinterpret_cast<float*>(hi_op + kPairE + kmajor_off(n, lane, N2)) = l;
-          }
-        }
-        __syncwarp();
-      }
+      build_pair_e<MR>(tk, e_op, Xp, Yp, warp, lane, kPairWarps);
     }
 #pragma unroll
     for (int i = 0; i < 16; ++i) acc[0][i] = acc[1][i] = 0.0;
@@ -584,6 +595,266 @@ __global__ void __launch_bounds__(tc::kPairThreads, 1)
                    long long tiles8, int blocks4) {
   if ((int)blockIdx.x < blocks4) pair_gram<MR, 4>(tasks, begins, n4, tiles4, blockIdx.x, (uint32_t)blocks4);
   else pair_gram<MR, 8>(tasks + n4, begins + n4, n8, tiles8, blockIdx.x - (uint32_t)blocks4, gridDim.x - (uint32_t)blocks4);
+}
+
+// ---------------------------------------------------------------------------
+// Both legs of a pair absorbed in one pass, out[x', y', o] =
+// sum_{x, y} in[x, y, o] E_x[x, x'] E_y[y, y']: the W of the site's other pair
+// (two absorptions of bp.h:137-152).
+//
+// Why: two launches of the leg kernel read and wrote the tensor twice; here it
+// is read and written once, which leaves HBM (64 KB per tile at D = 32, about
+// 2800 cycles per SM) and the two products' MMAs (1700 cycles) as bounds.
+// One 8x8 sweep at D = 32: 1.86 ms in the leg kernel, 1.15 ms here (6000
+// cycles per tile when planes are contiguous, 10700 when memory runs along o
+// and a tile is 32-byte pieces); 6x6 at D = 16: 0.09 -> 0.04 ms.
+//
+// Tiles, rows and tensor-memory operands are those of pair_gram.  The first
+// product's rows (o, x) go back over the tile they came from, the second
+// takes rows (o, y) from there, and its rows return to the same place, from
+// which the tile is written out as memory runs.  256 threads, two CTAs per SM
+// (98 KB of shared memory, 256 tensor-memory columns each): one converts
+// while the other waits.
+// ---------------------------------------------------------------------------
+namespace tc {
+constexpr int kAbsorbThreads = 512;
+constexpr uint32_t kAbsorbG = kAbsorbThreads / 128;  // warps that share a row
+__host__ __device__ constexpr size_t absorb_smem_bytes() {
+  return 1024 + 4 * (size_t)kPairE + 2 * (size_t)kPairRawElems * 8 + 64;
+}
+}  // namespace tc
+
+template <typename MR, uint32_t P>
+__device__ __forceinline__ void pair_absorb(const LegPairTask* __restrict__ tasks, const long long* __restrict__ begins, int ntask,
+                                            long long ntile_all, uint32_t block, uint32_t nblock) {
+  using namespace tc;
+  extern __shared__ __align__(1024) unsigned char pr_smem_raw[];
+  unsigned char* e_op = pr_smem_raw + ((1024 - (smem_u32(pr_smem_raw) & 1023)) & 1023);  // E_y hi, lo, E_x hi, lo
+  float2* raw = reinterpret_cast<float2*>(e_op + 4 * kPairE);                             // two tiles
+  uint64_t* bar = reinterpret_cast<uint64_t*>(raw + 2 * kPairRawElems);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const long long share = (ntile_all + nblock - 1) / nblock, first = block * share, last = min(ntile_all, first + share);
+  if (first >= last) return;
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(256u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(1u));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot, base = uniform(tmem);
+  constexpr uint32_t kColP = 128;  // A operand at 0, D1 at 128, D2 at 192
+
+  // rows: (o, x) or (o, y); of a row's groups of four columns, j, this warp
+  // has those with j % 4 == g
+  const int row = 32 * (warp & 3) + lane;
+  const uint32_t g = (uint32_t)warp >> 2, lanes = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+  // of the task: padded dimensions, this thread's place in a tile
+  uint32_t Xp = 8, Yp = 8, PE = 0, base_x = 0, base_y = 0, swz_y = 0;
+  // and its copies: the element (o, x) of every y = g + 4 k, at cp_d + y PE of
+  // a tile and at cp_off + y cp_step (cp_plane per unit of o / L1) in memory
+  uint32_t cp_o = 0, cp_d = 0, L1 = 1, Dy = 0, n_outer = 0;
+  bool cp_mine = false, cp_pad = false;
+  size_t cp_off = 0, cp_step = 0, cp_plane = 0;
+  FastDiv div_l{1, 1, 0};
+  const float2* src = nullptr;
+  ptrdiff_t dst = 0;  // output minus input
+
+  // offset at y = g of this thread's element in tile lt; false if it has none
+  auto place = [&](uint32_t lt, size_t& off) {
+    const uint32_t oo = lt * P + cp_o, hi = fast_div(oo, div_l);
+    off = cp_off + (oo - hi * L1) + cp_plane * hi;
+    return cp_mine && oo < n_outer;
+  };
+  auto load_tile = [&](uint32_t lt, int stage) {
+    if (cp_mine || cp_pad) {
+      size_t off;
+      const bool ok = place(lt, off);
+      const float2* p = ok ? src + off : src;
+      float2* d = raw + (size_t)stage * kPairRawElems + cp_d;
+#pragma unroll 4
+      for (uint32_t y = g; y < Yp; y += kAbsorbG) {
+        const bool in = ok && y < Dy;
+        cp8(d, in ? p : src, in);
+        p += cp_step;
+        d += kAbsorbG * PE;
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // rows of the tile as the A operand: [re_hi | im_hi | re_lo | im_lo]
+  auto put_a = [&](const float2* t, bool target_y) {
+    const uint32_t n = (target_y ? Xp : Yp) / 4;
+#pragma unroll
+    for (uint32_t j = g; j < 8; j += kAbsorbG)
+      if (j < n) {
+        const uint32_t step = target_y ? 1u : PE, c = lanes + 4 * j;
+        const float2* p = t + (target_y ? base_y + ((4 * j) ^ swz_y) : base_x + 4 * j * PE);
+        const float2 e0 = p[0], e1 = p[step], e2 = p[2 * step], e3 = p[3 * step];
+        float4 rh, rl, ih, il;
+        split4(make_float4(e0.x, e1.x, e2.x, e3.x), rh, rl);
+        split4(make_float4(e0.y, e1.y, e2.y, e3.y), ih, il);
+        tmem_st4(c, rh);
+        tmem_st4(c + 32u, ih);
+        tmem_st4(c + 64u, rl);
+        tmem_st4(c + 96u, il);
+      }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  };
+  // the product's rows back over the tile
+  auto put_back = [&](float2* t, bool target_y) {
+    const uint32_t Np = target_y ? Xp : Yp, n = Np / 4;
+    const bool valid = (uint32_t)row < P * (target_y ? Yp : Xp);
+#pragma unroll
+    for (uint32_t j = g; j < 8; j += kAbsorbG)
+      if (j < n) {
+        const uint32_t step = target_y ? 1u : PE, c = lanes + kColP + 4 * j;
+        float rr[4], ri[4], ir[4], ii[4];
+        tmem_ld4_async(c, rr);            // A_re E_re
+        tmem_ld4_async(c + Np, ri);       // A_re E_im
+        tmem_ld4_async(c + 64, ir);       // A_im E_re
+        tmem_ld4_async(c + 64 + Np, ii);  // A_im E_im
+        tmem_ld_wait16(rr, ri, ir, ii);
+        if (valid) {
+          float2* p = t + (target_y ? base_y + ((4 * j) ^ swz_y) : base_x + 4 * j * PE);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) p[k * step] = make_float2(rr[k] - ii[k], ri[k] + ir[k]);
+        }
+      }
+  };
+  auto leg_mma = [&](uint32_t which) {  // by warp 0; 0: E_y (K = Yp), 1: E_x
+    const uint32_t k8 = uniform(which ? Xp : Yp) / 8, N2 = 16 * k8, idesc = idesc_tf32(128, 0) | ((N2 >> 3) << 17);
+    const uint32_t op = uniform(smem_u32(e_op)) + which * 2 * kPairE;
+    const uint64_t dh0 = smem_desc(op, N2 * 16, 128), dl0 = smem_desc(op + kPairE, N2 * 16, 128);
+    if (elect_one()) {
+#pragma unroll
+      for (uint32_t part = 0; part < 2; ++part)
+#pragma unroll
+        for (uint32_t s = 0; s < 4; ++s)
+          if (s < k8) {
+            const uint32_t d = base + kColP + 64u * part, ah = base + 32u * part + 8u * s;
+            const uint64_t dh = dh0 + s * 2 * N2, dl = dl0 + s * 2 * N2;
+            mma_tf32_ts(d, ah, dh, idesc, s);
+            mma_tf32_ts(d, ah, dl, idesc, 1u);
+            mma_tf32_ts(d, ah + 64u, dh, idesc, 1u);
+          }
+      mma_commit(smem_u32(bar));
+    }
+    __syncwarp();
+  };
+  auto sync = [&]() {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  };
+  uint32_t phase = 0;
+  bool ok = true;
+  auto done = [&]() {  // every thread; the same answer for all
+    const bool r = mbar_wait(smem_u32(bar), phase);
+    phase ^= 1u;
+    ok = !__syncthreads_or(!r);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    return ok;
+  };
+
+  long long task_end = first;  // tile at which the current task ends
+  uint32_t lt = 0;
+  int ti = find_task(begins, ntask, first) - 1;
+  bool loaded = false;
+  for (long long tile = first; tile < last; ++tile, ++lt) {
+    const int stage = (int)(tile - first) & 1;
+    float2* t = raw + (size_t)stage * kPairRawElems;
+    if (tile == task_end) {  // the next task; its first tile is loaded below
+      const LegPairTask& tk = tasks[++ti];
+      const uint32_t Dx = (uint32_t)tk.Dx;
+      Dy = (uint32_t)tk.Dy;
+      L1 = (uint32_t)tk.L1;
+      n_outer = (uint32_t)tk.n_outer;
+      div_l = tk.div_l;
+      task_end = begins[ti] + (n_outer + P - 1) / P;
+      lt = (uint32_t)(tile - begins[ti]);
+      Xp = (Dx + 7u) & ~7u;
+      Yp = (Dy + 7u) & ~7u;
+      PE = (P * Xp) | 1u;
+      const uint32_t ox = (uint32_t)row / Xp, xx = (uint32_t)row - ox * Xp, oy = (uint32_t)row / Yp, yy = (uint32_t)row - oy * Yp;
+      base_x = ox < P ? ox * Xp + (xx ^ pair_swizzle(ox, Xp)) : 0;  // + y PE
+      base_y = oy < P ? yy * PE + oy * Xp : 0;                      // + (x ^ swz_y)
+      swz_y = pair_swizzle(oy, Xp);
+      // 32 elements (o, x) per instruction as memory runs: along x when the
+      // plane is contiguous, along o when consecutive o are
+      const uint32_t el = (uint32_t)row, o = L1 == 1 ? el / Xp : el % P, x = L1 == 1 ? el - o * Xp : el / P;
+      cp_o = o;
+      cp_mine = o < P && x < Dx;
+      cp_pad = o < P && x < Xp && !cp_mine;
+      cp_d = o * Xp + (x ^ pair_swizzle(o, Xp)) + g * PE;
+      cp_off = (size_t)L1 * (x + (size_t)Dx * g);
+      cp_step = (size_t)L1 * Dx * kAbsorbG;
+      cp_plane = (size_t)L1 * Dx * Dy;
+      src = static_cast<const float2*>(tk.V);
+      dst = static_cast<const float2*>(tk.W) - src;
+      loaded = false;
+      build_pair_e<MR>(tk, e_op, Xp, Yp, warp, lane, kAbsorbThreads / 32);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (!loaded) {
+      __syncthreads();  // the stage has been written out
+      load_tile(lt, stage);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // the tile is here; the other stage has been written out
+    loaded = tile + 1 < task_end && tile + 1 < last;
+    if (loaded) load_tile(lt + 1, stage ^ 1);
+    put_a(t, false);
+    sync();
+    if (warp == 0) leg_mma(0);
+    if (!done()) break;
+    put_back(t, false);
+    __syncthreads();
+    put_a(t, true);
+    sync();
+    if (warp == 0) leg_mma(1);
+    if (!done()) break;
+    put_back(t, true);
+    sync();
+    size_t off;
+    if (place(lt, off)) {
+      float2* out = const_cast<float2*>(src) + dst + off;
+      const float2* s = t + cp_d;
+#pragma unroll 4
+      for (uint32_t y = g; y < Dy; y += kAbsorbG) {
+        *out = *s;
+        out += cp_step;
+        s += kAbsorbG * PE;
+      }
+    }
+  }
+  if (!ok && tid == 0) {
+    // MMAs in flight get one more bounded wait before TMEM is freed
+    atomicExch(&g_tc_error, 1);
+    mbar_wait(smem_u32(bar), phase ^ 1u);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u));
+  }
+}
+
+// The tasks' `W` is the output.
+template <typename MR>
+__global__ void __launch_bounds__(tc::kAbsorbThreads, 2)
+    k_pair_absorb_tc(const LegPairTask* __restrict__ tasks, const long long* __restrict__ begins, int n4, long long tiles4, int n8,
+                     long long tiles8, int blocks4) {
+  if ((int)blockIdx.x < blocks4) pair_absorb<MR, 4>(tasks, begins, n4, tiles4, blockIdx.x, (uint32_t)blocks4);
+  else pair_absorb<MR, 8>(tasks + n4, begins + n4, n8, tiles8, blockIdx.x - (uint32_t)blocks4, gridDim.x - (uint32_t)blocks4);
 }
 
 }  // namespace tnbp

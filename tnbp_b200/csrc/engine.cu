@@ -34,6 +34,7 @@
 #include "tc_leg.cuh"
 #include "tc_leg_bulk.cuh"
 #include "tc_gram.cuh"
+#include "tc_gram64.cuh"
 #include "tc_leg64.cuh"
 #include "tc_leg_gram.cuh"
 #include "tc_pair.cuh"
@@ -1129,7 +1130,7 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
           } else if (tc_ok && tc::leg64_ok(lt.Din, lt.Dout)) {
             lt.block_begin = nb4;
             b4.push_back(nb4);
-            nb4 += (lt.L * lt.R + tc::kTcRows - 1) / tc::kTcRows;
+            nb4 += tc::leg64_tiles(lt.L, lt.R);
             t4.push_back(lt);
           } else if (tc_ok && lt.Din <= tc::kTcMaxD && lt.Dout <= tc::kTcMaxD) {
             lt.block_begin = nb2;
@@ -1277,9 +1278,9 @@ static int launch_batch_t(const SweepBatch& b, cudaStream_t stream) {
         break;
       }
       case SweepLaunch::LEG_T64: {
-        // persistent: one 256-thread CTA per SM (about 193 KB of shared memory)
+        // persistent: one CTA per SM
         const long long grid = std::min<long long>(L.nblocks, num_sms());
-        k_leg_apply_tc64<MR><<<(unsigned)grid, 256, tc::leg64_smem_bytes(), stream>>>(
+        k_leg_apply_tc64<MR><<<(unsigned)grid, tc::kLeg64Threads, tc::leg64_smem_bytes(), stream>>>(
             static_cast<const LegTask*>(tasks), begins, L.ntask, L.nblocks);
         break;
       }
@@ -1304,7 +1305,7 @@ static int launch_batch_t(const SweepBatch& b, cudaStream_t stream) {
             static_cast<const GramTask*>(tasks), begins, L.ntask);
         break;
       case SweepLaunch::GRAM_T64:
-        k_gram_tc64<<<(unsigned)L.nblocks, 256, tc::gram64_smem_bytes(), stream>>>(
+        k_gram_tc64<<<(unsigned)L.nblocks, tc::kGram64Threads, tc::gram64_smem_bytes(), stream>>>(
             static_cast<const GramTask*>(tasks), begins, L.ntask);
         break;
       case SweepLaunch::LEG_GRAM:

@@ -1,218 +1,312 @@
 // Leg contraction on tcgen05 for bond dimensions above 32 (chi = 32 requests
 // run BP at D = 64):  out[l, k, r] = sum_j in[l, j, r] * M[j, k],
-// complex64 tensors, 32 < max(Din, Dout) <= 64.
+// complex64 tensors, 32 < max(Din, Dout) <= 64, 3xTF32 as in k_leg_apply_tc.
 //
-// The product and the 3xTF32 split are those of k_leg_apply_tc
-// (tc_leg.cuh): real GEMM [A_re | A_im] (128 x 2Dp) x [[M_re, M_im],
-// [-M_im, M_re]] (2Dp x 2Dq).  With Dp, Dq up to 64 the operands no longer
-// fit shared memory at once, so K (2Dp <= 128) is walked in chunks of 64:
-// the message operand stays resident (N2 x K2, hi and lo: up to 128 KB), the
-// tile operand is built one K chunk at a time (128 x 64, hi and lo: 64 KB),
-// and the chunks' MMAs accumulate into one TMEM accumulator of N2 <= 128
-// columns.  256 threads, two per tile row: half h loads and converts
-// j in [32h, 32h + 32) and stores output columns [Dq h / 2, Dq (h+1) / 2);
-// warps w and w + 4 read TMEM lane quadrant w & 3.  The next tile's loads
-// are issued before the wait on the last chunk's MMAs.
+// What bounds it: at D = 64 a 128-row tile moves 128 KB, about 5600 cycles of
+// an SM's share of HBM, and its MMAs take 3100.  The kernel before this one
+// converted straight from global loads into shared-memory operands with one
+// tile in flight and waited for every chunk's MMAs (23000 cycles per tile).
+// Here a tile arrives by cp.async while the one before it is worked on; its
+// rows go to tensor memory as the A operand (shared memory then holds only
+// M: [M_re | M_im], D1 = A_re M', D2 = A_im M'), K in two halves with an
+// operand each, so that the next tile's first half is converted during this
+// tile's second MMAs; the result returns over the tile it came from and is
+// written out as memory runs.  Per 5x5 sweep at D = 64: 24.9 -> 10.8 ms (9000
+// cycles per tile, 4 TB/s; 11000 at L = 1, whose tiles go out through shared
+// memory).
 //
-// Every wait is bounded: on timeout the CTA records g_tc_error, waits once
-// more (bounded) for its MMAs, frees its TMEM and returns.
+// 512 threads, persistent, one CTA per SM (194 KB of shared memory, all of
+// tensor memory).  Every wait is bounded: on timeout the CTA records
+// g_tc_error, waits once more (bounded) for its MMAs, frees its TMEM and
+// returns.
 #pragma once
 #include <cstdint>
 
-#include "tc_leg.cuh"
+#include "tc_pair.cuh"
 
 namespace tnbp {
 namespace tc {
 
 constexpr int kTcMaxD64 = 64;
-constexpr int kChunkK = 64;  // real K per chunk
+constexpr int kLeg64Threads = 512;
+constexpr int kLeg64Pitch = kTcRows + 1;  // element (row, j) of a tile at j pitch + row: odd
+constexpr uint32_t kLeg64Op = 128 * 64 * 4;
 
 __host__ __device__ constexpr size_t leg64_smem_bytes() {
-  // A chunk (hi, lo): 128 x 64 fp32 each; B (hi, lo): 128 x 128 fp32 each
-  return 1024 + (size_t)2 * kTcRows * kChunkK * 4 + (size_t)2 * (2 * kTcMaxD64) * (2 * kTcMaxD64) * 4 + 64;
+  return 1024 + 2 * (size_t)kLeg64Op + 2 * (size_t)kTcMaxD64 * kLeg64Pitch * 8 + 64;
 }
 __host__ __device__ inline bool leg64_ok(int Din, int Dout) {
   return Din <= kTcMaxD64 && Dout <= kTcMaxD64 && (Din > kTcMaxD || Dout > kTcMaxD);
+}
+// Rows per tile: whole (l, j) blocks for L <= 32, so that the tile is one
+// contiguous range of memory; above that 128, each run of l contiguous.
+__host__ __device__ inline int leg64_rows(long long L) { return L <= 32 ? (int)(kTcRows / L * L) : kTcRows; }
+__host__ __device__ inline long long leg64_tiles(long long L, long long R) {
+  const long long rows = leg64_rows(L);
+  return (L * R + rows - 1) / rows;
 }
 
 }  // namespace tc
 
 template <typename MR>
-__global__ void __launch_bounds__(256) k_leg_apply_tc64(const LegTask* __restrict__ tasks,
-                                                        const long long* __restrict__ begins, int ntask,
-                                                        long long total_tiles) {
+__global__ void __launch_bounds__(tc::kLeg64Threads, 1) k_leg_apply_tc64(const LegTask* __restrict__ tasks,
+                                                                        const long long* __restrict__ begins, int ntask,
+                                                                        long long total_tiles) {
   using namespace tc;
   extern __shared__ __align__(1024) unsigned char t64_smem_raw[];
-  unsigned char* smem = t64_smem_raw + ((1024 - (smem_u32(t64_smem_raw) & 1023)) & 1023);
-  unsigned char* a_hi = smem;                                    // 128 x 64 fp32
-  unsigned char* a_lo = a_hi + kTcRows * kChunkK * 4;
-  unsigned char* b_hi = a_lo + kTcRows * kChunkK * 4;            // up to 128 x 128 fp32
-  unsigned char* b_lo = b_hi + (2 * kTcMaxD64) * (2 * kTcMaxD64) * 4;
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(b_lo + (2 * kTcMaxD64) * (2 * kTcMaxD64) * 4);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar + 1);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int row = tid & 127, half = tid >> 7;
-  constexpr int kHalfD = kTcMaxD64 / 2;  // j per thread
-
-  const long long per = (total_tiles + gridDim.x - 1) / gridDim.x;
-  const long long t_begin = (long long)blockIdx.x * per;
-  const long long t_end = min(total_tiles, t_begin + per);
-  if (t_begin >= t_end) return;
+  unsigned char* b_op = t64_smem_raw + ((1024 - (smem_u32(t64_smem_raw) & 1023)) & 1023);  // M: hi, lo
+  float2* raw = reinterpret_cast<float2*>(b_op + 2 * kLeg64Op);                             // two tiles
+  // per half: operand written, MMAs done; per tile parity: tile arrived
+  uint64_t* bars = reinterpret_cast<uint64_t*>(raw + 2 * kTcMaxD64 * kLeg64Pitch);
+  const uint32_t bar_ready = smem_u32(bars), bar_done = bar_ready + 16, bar_full = bar_ready + 32;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
+  volatile int* fail = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const long long per = (total_tiles + gridDim.x - 1) / gridDim.x, first = blockIdx.x * per, last = min(total_tiles, first + per);
+  if (first >= last) return;
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(128u));
+                 "r"(512u));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar)), "r"(1u));
+    for (int i = 0; i < 6; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bars + i)),
+                   "r"(i < 2 ? kLeg64Threads / 32u : i < 4 ? 1u : (uint32_t)kLeg64Threads));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    *fail = 0;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = *tmem_slot, base = uniform(tmem);
+  constexpr uint32_t kColD = 256;  // A halves at 0 and 128 ([re_hi | im_hi | re_lo | im_lo] of 32 columns), D1 at 256, D2 at 384
 
-  float2 nxt[kHalfD];
-  // this thread's half of one tile row (j in [32 half, 32 half + 32)) into
-  // registers; rows < 2^31, 32-bit row split
-  auto load_row = [&](long long tile, int task_id) {
-    const LegTask t = tasks[task_id];
-    const unsigned q = (unsigned)((tile - t.block_begin) * kTcRows) + (unsigned)row;
-    const unsigned rows = (unsigned)(t.L * t.R), L = (unsigned)t.L;
-    const int j0 = kHalfD * half;
-    if (q < rows && j0 < t.Din) {
-      const unsigned l = q % L, r = q / L;
-      const float2* __restrict__ p =
-          static_cast<const float2*>(t.in) + (size_t)l + (size_t)L * ((size_t)t.Din * r + j0);
-#pragma unroll
-      for (int j = 0; j < kHalfD; ++j) nxt[j] = j0 + j < t.Din ? __ldg(p + (size_t)L * j) : make_float2(0.f, 0.f);
-    } else {
-#pragma unroll
-      for (int j = 0; j < kHalfD; ++j) nxt[j] = make_float2(0.f, 0.f);
+  const int row = 32 * (warp & 3) + lane;
+  const uint32_t g = (uint32_t)warp >> 2;  // groups of four columns, j: those with j % 4 == g
+  const uint32_t lanes = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+
+  // of the current task
+  LegTask tk{};
+  uint32_t L = 1, rows = 0, rpt = kTcRows, Din = 0, Dout = 0, Np = 8, nk = 1, nk0 = 1;  // K steps of 8, of the first half
+
+  auto load_tile = [&](uint32_t lt, int stage) {
+    float2* d = raw + (size_t)stage * kTcMaxD64 * kLeg64Pitch;
+    const float2* in = static_cast<const float2*>(tk.in);
+    const uint32_t q0 = lt * rpt, n = min(rpt, rows - q0);
+    if (L <= 32) {
+      const float2* p = in + (size_t)q0 * Din;
+      for (uint32_t i = (uint32_t)tid; i < n * Din; i += kLeg64Threads) {
+        const uint32_t c = fast_div(i, tk.div_l), l = i - c * L, r = fast_div(c, tk.div_din), j = c - r * Din;
+        cp8(d + j * kLeg64Pitch + r * L + l, p + i, true);
+      }
+    } else if ((uint32_t)row < n) {
+      const uint32_t q = q0 + (uint32_t)row, r = fast_div(q, tk.div_l), l = q - r * L;
+      const float2* p = in + (size_t)l + (size_t)L * ((size_t)Din * r + g);
+      float2* e = d + g * kLeg64Pitch + row;
+#pragma unroll 4
+      for (uint32_t j = g; j < Din; j += 4) {
+        cp8(e, p, true);
+        p += (size_t)L * 4;
+        e += 4 * kLeg64Pitch;
+      }
     }
+    // this thread's arrival, when its copies have landed
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar_full + 8u * stage) : "memory");
   };
-
-  int cur_task = -1;
-  LegTask tk;
-  int Din = 0, Dout = 0, Dp = 4, Dq = 8;
-  int task_of_next = find_task(begins, ntask, t_begin);
-  load_row(t_begin, task_of_next);
-  uint32_t phase = 0;
-  bool failed = false;
-  for (long long tile = t_begin; tile < t_end && !failed; ++tile) {
-    const int task_id = task_of_next;
-    if (task_id != cur_task) {  // the previous tile's MMAs completed: B is free
-      cur_task = task_id;
-      tk = tasks[task_id];
-      Din = tk.Din;
-      Dout = tk.Dout;
-      Dp = (Din + 3) & ~3;
-      Dq = (Dout + 7) & ~7;
-      const int K2 = 2 * Dp, N2 = 2 * Dq;
-      const typename cvec<MR>::type* __restrict__ mat = static_cast<const typename cvec<MR>::type*>(tk.mat);
-      // B_real[k2][n2] = [[M_re, M_im], [-M_im, M_re]], stored N2 x K2 K-major
-      for (int n2 = warp; n2 < N2; n2 += 8) {
-        const int nr = n2 < Dq ? n2 : n2 - Dq, pn = n2 < Dq ? 0 : 1;
-        for (int k2 = lane; k2 < K2; k2 += 32) {
-          const int kr = k2 < Dp ? k2 : k2 - Dp, pk = k2 < Dp ? 0 : 1;
-          double v = 0.0;
-          if (kr < Din && nr < Dout) {
-            const double2 m = to_d2(mat[kr + (long long)Din * nr]);
-            v = (pk == pn) ? m.x : (pk == 0 ? m.y : -m.y);
+  auto put_a = [&](const float2* t, uint32_t half) {
+    const uint32_t j0 = half ? 2 * nk0 : 0, n = 2 * (half ? nk - nk0 : nk0);  // groups
+    const uint32_t a = lanes + 128 * half;
+#pragma unroll
+    for (uint32_t i = g; i < 8; i += 4)
+      if (i < n) {
+        const uint32_t j = 4 * (j0 + i);
+        const float2* p = t + j * kLeg64Pitch + row;
+        float2 e[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) e[k] = j + k < Din ? p[k * kLeg64Pitch] : make_float2(0.f, 0.f);
+        float4 rh, rl, ih, il;
+        split4(make_float4(e[0].x, e[1].x, e[2].x, e[3].x), rh, rl);
+        split4(make_float4(e[0].y, e[1].y, e[2].y, e[3].y), ih, il);
+        tmem_st4(a + 4 * i, rh);
+        tmem_st4(a + 4 * i + 32u, ih);
+        tmem_st4(a + 4 * i + 64u, rl);
+        tmem_st4(a + 4 * i + 96u, il);
+      }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  };
+  auto mma_half = [&](uint32_t half) {  // by warp 0
+    const uint32_t N2 = uniform(2 * Np), s0 = uniform(half ? nk0 : 0), n = uniform(half ? nk - nk0 : nk0);
+    const uint32_t idesc = idesc_tf32(128, 0) | ((N2 >> 3) << 17), op = uniform(smem_u32(b_op));
+    const uint64_t dh0 = smem_desc(op, N2 * 16, 128) + s0 * 2 * N2, dl0 = smem_desc(op + kLeg64Op, N2 * 16, 128) + s0 * 2 * N2;
+    if (elect_one()) {
+#pragma unroll
+      for (uint32_t part = 0; part < 2; ++part)
+#pragma unroll
+        for (uint32_t s = 0; s < 4; ++s)
+          if (s < n) {
+            const uint32_t d = base + kColD + 128u * part, ah = base + 128u * half + 32u * part + 8u * s;
+            const uint64_t dh = dh0 + s * 2 * N2, dl = dl0 + s * 2 * N2;
+            mma_tf32_ts(d, ah, dh, idesc, half + s);
+            mma_tf32_ts(d, ah, dl, idesc, 1u);
+            mma_tf32_ts(d, ah + 64u, dh, idesc, 1u);
           }
-          const float h = to_tf32((float)v), lo = to_tf32((float)(v - (double)h));
-          *reinterpret_cast<float*>(b_hi + kmajor_off(n2, k2, N2)) = h;
-          *reinterpret_cast<float*>(b_lo + kmajor_off(n2, k2, N2)) = lo;
-        }
-      }
+      mma_commit(bar_done + 8u * half);
     }
-    const int K2 = 2 * Dp, N2 = 2 * Dq;
-    const int nchunk = (K2 + kChunkK - 1) / kChunkK;
-    const uint32_t row_off = (uint32_t)((row >> 3) * 128 + (row & 7) * 16);
-    for (int ch = 0; ch < nchunk; ++ch) {
-      const int kc0 = ch * kChunkK, kcn = min(kChunkK, K2 - kc0);
-      // operand chunk: K2 index x = j (re) or Dp + j (im); groups of 4 j
-#pragma unroll
-      for (int g = 0; g < kHalfD / 4; ++g) {
-        const int j = kHalfD * half + 4 * g;  // first j of the group
-        if (j >= Dp) continue;
-#pragma unroll
-        for (int part = 0; part < 2; ++part) {
-          const int x = part * Dp + j;  // K2 index of the group
-          if (x < kc0 || x >= kc0 + kcn) continue;
-          float4 v;
-          float* pv = &v.x;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) pv[i] = part == 0 ? nxt[4 * g + i].x : nxt[4 * g + i].y;
-          const float4 h = make_float4(to_tf32(v.x), to_tf32(v.y), to_tf32(v.z), to_tf32(v.w));
-          const float4 lo = make_float4(to_tf32(v.x - h.x), to_tf32(v.y - h.y), to_tf32(v.z - h.z),
-                                        to_tf32(v.w - h.w));
-          const uint32_t o = (uint32_t)((x - kc0) >> 2) * (kTcRows * 16) + row_off;
-          *reinterpret_cast<float4*>(a_hi + o) = h;
-          *reinterpret_cast<float4*>(a_lo + o) = lo;
-        }
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncthreads();
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (tid == 0) {
-        const uint32_t idesc = idesc_tf32(kTcRows, N2);
-        const uint32_t a_lbo = kTcRows * 16, b_lbo = N2 * 16;
-        const uint32_t ah = smem_u32(a_hi), al = smem_u32(a_lo);
-        const uint32_t bh = smem_u32(b_hi) + (uint32_t)(kc0 >> 2) * b_lbo, bl = smem_u32(b_lo) + (uint32_t)(kc0 >> 2) * b_lbo;
-        for (int s = 0; s < kcn / 8; ++s) {
-          const uint32_t ao = (uint32_t)s * 2 * a_lbo, bo = (uint32_t)s * 2 * b_lbo;
-          const uint32_t acc0 = (ch > 0 || s > 0) ? 1u : 0u;
-          mma_tf32(tmem, smem_desc(ah + ao, a_lbo, 128), smem_desc(bh + bo, b_lbo, 128), idesc, acc0);
-          mma_tf32(tmem, smem_desc(ah + ao, a_lbo, 128), smem_desc(bl + bo, b_lbo, 128), idesc, 1u);
-          mma_tf32(tmem, smem_desc(al + ao, a_lbo, 128), smem_desc(bh + bo, b_lbo, 128), idesc, 1u);
-        }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                         smem_u32(mbar))
-                     : "memory");
-      }
-      if (ch + 1 == nchunk && tile + 1 < t_end) {  // next tile's loads during the last chunk's MMAs
-        task_of_next = (tile + 1 >= tk.block_begin + ((tk.L * tk.R + kTcRows - 1) / kTcRows))
-                           ? find_task(begins, ntask, tile + 1)
-                           : task_id;
-        load_row(tile + 1, task_of_next);
-      }
-      const bool ok = mbar_wait(smem_u32(mbar), phase);
-      if (__syncthreads_or(!ok)) {
-        if (tid == 0) atomicExch(&g_tc_error, 1);
-        if (!ok) mbar_wait(smem_u32(mbar), phase);
-        failed = true;
-        break;
-      }
-      phase ^= 1u;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncwarp();
+  };
+  // Warps meet only through barriers.  A bounded wait by a whole warp; false
+  // (for the whole warp) when it or any other warp gave up.
+  auto wait = [&](uint32_t bar, uint32_t phase) -> bool {
+    bool r = __all_sync(0xffffffffu, mbar_try(bar, phase));
+    for (int i = 0; i < kPairWaitLimit && !r; ++i) {
+      r = __all_sync(0xffffffffu, mbar_try(bar, phase));
+      if (!r && (i & 1023) == 1023 && __any_sync(0xffffffffu, *fail)) break;
     }
-    if (failed) break;
-    // epilogue: row's output columns n in [Dq h / 2, Dq (h+1) / 2): re in
-    // TMEM column n, im in column Dq + n
-    const int nh = Dq / 2, n0 = nh * half;
-    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    float cre[32], cim[32];
-    tmem_ld32(lane_addr + (uint32_t)n0, cre);
-    tmem_ld32(lane_addr + (uint32_t)(Dq + n0), cim);
-    const unsigned q = (unsigned)((tile - tk.block_begin) * kTcRows) + (unsigned)row;
-    if (q < (unsigned)(tk.L * tk.R)) {
-      const unsigned L = (unsigned)tk.L, l = q % L, r = q / L;
-      float2* __restrict__ p = static_cast<float2*>(tk.out) + (size_t)l + (size_t)L * ((size_t)Dout * r + n0);
-#pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (i < nh && n0 + i < Dout) p[(size_t)L * i] = make_float2(cre[i], cim[i]);
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    if (!r) *fail = 1;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    return r;
+  };
+  // this warp's part of a half's operand is written (and the last tile's D
+  // read); warp 0 issues when every warp's is
+  uint32_t ready_ph[2] = {0u, 0u}, done_ph[2] = {0u, 0u}, full_ph[2] = {0u, 0u};
+  auto publish = [&](uint32_t half) -> bool {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar_ready + 8u * half);
+    if (warp != 0) return true;
+    if (!wait(bar_ready + 8u * half, half ? ready_ph[1] : ready_ph[0])) return false;
+    if (half) ready_ph[1] ^= 1u; else ready_ph[0] ^= 1u;
+    mma_half(half);
+    return true;
+  };
+  auto done = [&](uint32_t half) {
+    const bool r = wait(bar_done + 8u * half, half ? done_ph[1] : done_ph[0]);
+    if (half) done_ph[1] ^= 1u; else done_ph[0] ^= 1u;
+    return r;
+  };
+  auto arrived = [&](int stage) {
+    const bool r = wait(bar_full + 8u * stage, stage ? full_ph[1] : full_ph[0]);
+    if (stage) full_ph[1] ^= 1u; else full_ph[0] ^= 1u;
+    return r;
+  };
+  bool ok = true;
+
+  int ti = find_task(begins, ntask, first) - 1;
+  long long task_end = first;
+  uint32_t lt = 0;
+  bool loaded = false;   // this tile's copies are on their way
+  bool halved = false;   // and its first half is in tensor memory
+  for (long long tile = first; tile < last; ++tile, ++lt) {
+    const int stage = (int)(tile - first) & 1;
+    float2* t = raw + (size_t)stage * kTcMaxD64 * kLeg64Pitch;
+    float2* t2 = raw + (size_t)(stage ^ 1) * kTcMaxD64 * kLeg64Pitch;
+    if (tile == task_end) {  // the next task: this warp waited for the last one's MMAs
+      tk = tasks[++ti];
+      L = (uint32_t)tk.L;
+      rows = (uint32_t)(tk.L * tk.R);
+      rpt = (uint32_t)leg64_rows(tk.L);
+      Din = (uint32_t)tk.Din;
+      Dout = (uint32_t)tk.Dout;
+      Np = (Dout + 7u) & ~7u;
+      nk = (Din + 7u) / 8;
+      nk0 = (nk + 1) / 2;
+      task_end = begins[ti] + leg64_tiles(tk.L, tk.R);
+      lt = (uint32_t)(tile - begins[ti]);
+      loaded = halved = false;
+      // element (n, k) of 2 Np rows (re, im), K = 8 nk columns
+      const typename cvec<MR>::type* __restrict__ mat = static_cast<const typename cvec<MR>::type*>(tk.mat);
+      for (uint32_t n = (uint32_t)warp; n < 2 * Np; n += kLeg64Threads / 32)
+        for (uint32_t k = (uint32_t)lane; k < 8 * nk; k += 32) {
+          const uint32_t c = n < Np ? n : n - Np;
+          double v = 0.0;
+          if (k < Din && c < Dout) {
+            const double2 m = to_d2(mat[k + (size_t)Din * c]);
+            v = n < Np ? m.x : m.y;
+          }
+          // the remainder in FP64, so that complex128 messages keep their low bits
+          const float h = to_tf32((float)v), l = to_tf32((float)(v - (double)h));
+          *reinterpret_cast<float*>(b_op + kmajor_off((int)n, (int)k, (int)(2 * Np))) = h;
+          *reinterpret_cast<float*>(b_op + kLeg64Op + kmajor_off((int)n, (int)k, (int)(2 * Np))) = l;
+        }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    // A stage is free once the MMAs of its tile are done (every warp has read
+    // it by then) or, where results go back over it, after the barrier below.
+    if (!loaded) load_tile(lt, stage);
+    const bool more = tile + 1 < task_end && tile + 1 < last;
+    if (!halved) {
+      if (!(ok = arrived(stage))) break;
+      put_a(t, 0);
+    }
+    if (!(ok = publish(0))) break;
+    if (more) load_tile(lt + 1, stage ^ 1);
+    loaded = more;
+    if (nk > nk0) {
+      put_a(t, 1);
+      if (!(ok = publish(1))) break;
+    }
+    if (!(ok = done(0))) break;
+    // the next tile's first half, during this one's second MMAs
+    halved = more;
+    if (more) {
+      if (!(ok = arrived(stage ^ 1))) break;
+      put_a(t2, 0);
+    }
+    if (nk > nk0 && !(ok = done(1))) break;
+    // D1, D2 of this row: back over the tile (both halves were read), or
+    // straight out where lanes run along memory
+    const uint32_t q0 = lt * rpt, n = min(rpt, rows - q0);
+    const bool direct = L > 32;
+    float2* out = static_cast<float2*>(tk.out);
+    size_t off = 0;
+    if (direct) {
+      const uint32_t q = q0 + (uint32_t)row, r = fast_div(q, tk.div_l), l = q - r * L;
+      off = (size_t)l + (size_t)L * (size_t)Dout * r;
+    }
+#pragma unroll
+    for (uint32_t i = g; i < 16; i += 4)
+      if (4 * i < Np) {
+        float rr[4], ri[4], ir[4], ii[4];
+        const uint32_t c = lanes + kColD + 4 * i;
+        tmem_ld4_async(c, rr);             // A_re M_re
+        tmem_ld4_async(c + Np, ri);        // A_re M_im
+        tmem_ld4_async(c + 128, ir);       // A_im M_re
+        tmem_ld4_async(c + 128 + Np, ii);  // A_im M_im
+        tmem_ld_wait16(rr, ri, ir, ii);
+        if ((uint32_t)row < n) {
+#pragma unroll
+          for (uint32_t k = 0; k < 4; ++k) {
+            const float2 v = make_float2(rr[k] - ii[k], ri[k] + ir[k]);
+            if (!direct) t[(4 * i + k) * kLeg64Pitch + row] = v;
+            else if (4 * i + k < Dout) out[off + (size_t)L * (4 * i + k)] = v;
+          }
+        }
+      }
+    if (!direct) {
+      __syncthreads();
+      float2* o = out + (size_t)q0 * Dout;
+      for (uint32_t i = (uint32_t)tid; i < n * Dout; i += kLeg64Threads) {
+        const uint32_t c = fast_div(i, tk.div_l), l = i - c * L;
+        const uint32_t r = Dout == Din ? fast_div(c, tk.div_din) : c / Dout, k = c - r * Dout;
+        o[i] = t[k * kLeg64Pitch + r * L + l];
+      }
+      __syncthreads();
+    }
+  }
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  if (*fail && tid == 0) {
+    // MMAs in flight get one more bounded wait before TMEM is freed
+    atomicExch(&g_tc_error, 1);
+    for (uint32_t i = 0; i < 4; ++i) mbar_wait(bar_done + 8u * (i >> 1), i & 1u);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128u));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
   }
 }
 

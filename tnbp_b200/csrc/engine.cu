@@ -876,12 +876,13 @@ void Job::build_plan() {
         g1.L = L; g1.M = M; g1.D = sh[t]; g1.P = 1; g1.C = sh[t];
         g1.ctiles = (g1.C + kColTile - 1) / kColTile;
         g1.Q = L * M;
-        // chunks of about Q/16 rows (multiples of 64, 256..4096): FP64
+        // chunks of about Q/16 rows (multiples of 64, 256..4096; up to 16384
+        // for more than 32 columns, whose partials are 64 KB each): FP64
         // partials of one sweep stay a small fraction of its traffic, and
         // one wave of all sites gives every SM work.  The chunking does not
         // depend on the wave budget, so neither does the rounding.
         long long cr = ((g1.Q / 16) + 63) / 64 * 64;
-        cr = std::max<long long>(256, std::min<long long>(4096, cr));
+        cr = std::max<long long>(256, std::min<long long>(g1.C > 32 ? 16384 : 4096, cr));
         g1.chunk_rows = cr;
         g1.nchunk = (int)((g1.Q + cr - 1) / cr);
         g1.partial = nullptr;
@@ -1331,7 +1332,7 @@ static int launch_batch_t(const SweepBatch& b, cudaStream_t stream) {
           k_gram<R><<<(unsigned)L.nblocks, kThreads, 0, stream>>>(static_cast<const GramTask*>(tasks), begins, L.ntask);
         break;
       case SweepLaunch::MSG:
-        k_msg_finalize<R, MR><<<L.ntask, kThreads, 0, stream>>>(static_cast<const MsgTask*>(tasks));
+        k_msg_finalize<R, MR><<<L.ntask, kFinalizeThreads, 0, stream>>>(static_cast<const MsgTask*>(tasks));
         break;
       case SweepLaunch::SITE:  // max_din holds the launch's shared memory bytes
         k_site_sweep<R, MR><<<L.ntask, kThreads, (size_t)L.max_din, stream>>>(static_cast<const SiteTask*>(tasks));
@@ -1601,7 +1602,6 @@ Tpo::~Tpo() {}
 
 void Job::absorb_tpo(const Tpo& tpo) {
   TNBP_TRACE_SCOPE("absorb");
-  shadow_dirty = true;
   const int ns = (int)g.labels.size();
   const int ne = (int)g.edges.size();
   if ((int)tpo.rank.size() != ne) throw Error(TNBP_EINVAL, "TPO edge count mismatch");
@@ -1617,6 +1617,20 @@ void Job::absorb_tpo(const Tpo& tpo) {
   nV.ensure(v_elems * esz, stream);
   nM0.alloc(m_elems * esz, stream);
   nM1.alloc(m_elems * esz, stream);
+  plan.valid = false;
+  destroy_graphs();
+  plan = SweepPlan();  // it holds the old addresses
+  // the mixed path's complex64 copy is written along if it fits now, else
+  // before the first sweep (sync_shadow)
+  bool along = prec == TNBP_MIXED &&
+               !(budget && device_bytes() - V32.bytes + std::max<uint64_t>(V32.bytes, v_elems * 8) > budget);
+  if (along) {
+    try {
+      V32.ensure(v_elems * 8, stream);
+    } catch (const Error&) {
+      along = false;
+    }
+  }
   std::vector<AbsorbTask> at;
   std::vector<long long> ab;
   long long nb = 0;
@@ -1627,18 +1641,21 @@ void Job::absorb_tpo(const Tpo& tpo) {
     t.O = static_cast<const double2*>(tpo.ops.p) + tpo.op_offset[s];
     t.g = (int)g.legs[s].size();
     t.d = pd[s];
-    t.dout = tpo.dout[s];
+    t.out32 = along ? static_cast<float2*>(V32.p) + voff[s] : nullptr;
+    t.nv = 1;
+    t.ncombo = t.d;
     for (int k = 0; k < t.g; ++k) {
       t.Dv[k] = odim[g.legs[s][k]];
       t.r[k] = tpo.rank[g.legs[s][k]];
-      t.div_m[k] = make_fastdiv((uint32_t)(t.Dv[k] * t.r[k]));
       t.div_v[k] = make_fastdiv((uint32_t)t.Dv[k]);
+      t.nv *= t.Dv[k];
+      t.ncombo *= t.r[k];
     }
-    t.n_out = (long long)site_elems(s);
-    if (t.n_out >= (1ll << 31)) throw Error(TNBP_EUNSUPPORTED, "site tensor of 2^31 or more elements");
+    if ((long long)site_elems(s) >= (1ll << 31)) throw Error(TNBP_EUNSUPPORTED, "site tensor of 2^31 or more elements");
+    t.vblocks = (int)((t.nv + kThreads - 1) / kThreads);
     t.block_begin = nb;
     ab.push_back(nb);
-    nb += (t.n_out + kThreads - 1) / kThreads;
+    nb += (long long)t.vblocks * ((t.ncombo + kAbsorbCombos - 1) / kAbsorbCombos);
     at.push_back(t);
   }
   std::vector<MsgExpandTask> mt;
@@ -1669,13 +1686,11 @@ void Job::absorb_tpo(const Tpo& tpo) {
     (k_expand_msgs<float><<<(unsigned)nmb, kThreads, 0, stream>>>(static_cast<MsgExpandTask*>(dmt.p), static_cast<long long*>(dmb.p), (int)mt.size()), note_launch());
   }
   CK(cudaGetLastError());
+  shadow_dirty = !along;
   std::swap(V, nV);
   std::swap(M[0], nM0);
   std::swap(M[1], nM1);
   cur = 0;
-  plan.valid = false;
-  destroy_graphs();
-  plan = SweepPlan();
   CK(cudaStreamSynchronize(stream));
   check_budget();
 }

@@ -305,7 +305,7 @@ constexpr size_t kSiteSmemMax = 64 * 1024;
 // stored message (bp.h:341-350).  One block per message.
 // ---------------------------------------------------------------------------
 struct MsgTask {
-  const double2* partial;
+  double2* partial;  // [nchunk][C * C], the first chunk is overwritten
   int nchunk, C;
   void* out;        // new message (C x C), storage precision
   const void* old;  // stored message (same dim) or nullptr
@@ -329,18 +329,24 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   return red[0];
 }
 
-// OR: element type of the stored messages (out and old).
+// OR: element type of the stored messages (out and old).  The chunks are read
+// once: their sum replaces the first one, from which the second pass
+// normalizes (reading them again took half of the time, 0.70 ms per 5x5 sweep
+// at D = 64; 0.11 ms with 512 threads and chunks of 16384 rows there).
+constexpr int kFinalizeThreads = 512;
 template <typename R, typename OR = R>
-__global__ void __launch_bounds__(kThreads) k_msg_finalize(const MsgTask* __restrict__ tasks) {
+__global__ void __launch_bounds__(kFinalizeThreads) k_msg_finalize(const MsgTask* __restrict__ tasks) {
   using C = typename cvec<OR>::type;
   __shared__ double red[32];
   const MsgTask tk = tasks[blockIdx.x];
   const int n = tk.C * tk.C;
   const C* old = static_cast<const C*>(tk.old);
   double s_new = 0.0, s_old = 0.0;
-  for (int i = threadIdx.x; i < n; i += kThreads) {
+  for (int i = threadIdx.x; i < n; i += kFinalizeThreads) {
     double2 v = make_double2(0.0, 0.0);
+#pragma unroll 8
     for (int c = 0; c < tk.nchunk; ++c) v = v + tk.partial[(long long)c * n + i];
+    tk.partial[i] = v;
     s_new += abs2(v);
     if (old) s_old += abs2(to_d2(old[i]));
   }
@@ -350,10 +356,8 @@ __global__ void __launch_bounds__(kThreads) k_msg_finalize(const MsgTask* __rest
   const double inv_o = no > 0.0 ? 1.0 / no : 1.0;
   double d2 = 0.0;
   C* out = static_cast<C*>(tk.out);
-  for (int i = threadIdx.x; i < n; i += kThreads) {
-    double2 v = make_double2(0.0, 0.0);
-    for (int c = 0; c < tk.nchunk; ++c) v = v + tk.partial[(long long)c * n + i];
-    v = inv_n * v;
+  for (int i = threadIdx.x; i < n; i += kFinalizeThreads) {
+    const double2 v = inv_n * tk.partial[i];
     if (old) d2 += abs2(v - inv_o * to_d2(old[i]));
     out[i] = from_d2<C>(v);
   }
@@ -402,52 +406,89 @@ static __global__ void k_sum_scaled(const double* __restrict__ x, int n, double 
 // AbsorbTPO, site part (apply.h:43-66):
 //   V'[(v_0,o_0),...,(v_{g-1},o_{g-1}), p'] = sum_p O[o..., p, p'] V[v..., p]
 // merged bond index v + D*o (column-major reshape of (v, o)).
+//
+// A thread owns one v = (v_0, ..., v_{g-1}): it splits that index once, reads
+// V[v, :] once and writes the element of every o and p' of its block (`combo`,
+// with the operator's values and the output offsets in shared memory), lanes
+// along v_0.  One thread per output element spent its time splitting indices:
+// 12x12 from D = 16 to 32 (3.6 GB written) 2.65 ms, here 0.81 ms with the
+// complex64 copy the mixed path's sweeps read (out32, may be null), which was
+// a pass of its own of 0.75 ms.
 // ---------------------------------------------------------------------------
+constexpr int kAbsorbCombos = 128;  // (o, p') of one block
 struct AbsorbTask {
   const void* V;
   void* out;
+  float2* out32;
   const double2* O;  // op tensor (r_0..r_{g-1}, d, d'), complex128
-  int g, d, dout;
+  int g, d;
   int Dv[kMaxLegs];
   int r[kMaxLegs];
-  FastDiv div_m[kMaxLegs];  // by Dv[k] r[k] (the merged bond of leg k)
   FastDiv div_v[kMaxLegs];  // by Dv[k]
-  long long n_out;          // < 2^31 (checked on the host)
+  long long nv;             // prod Dv; the output, nv ncombo, < 2^31 elements (checked on the host)
+  long long ncombo;         // prod r d
+  int vblocks;              // blocks along v; the others run along combos
   long long block_begin;
 };
-
 template <typename R>
 __global__ void __launch_bounds__(kThreads) k_absorb_sites(const AbsorbTask* __restrict__ tasks,
                                                            const long long* __restrict__ begins,
                                                            int ntask) {
   using C = typename cvec<R>::type;
-  const int ti = find_task(begins, ntask, blockIdx.x);
-  const AbsorbTask& tk = tasks[ti];
-  const long long i = (blockIdx.x - tk.block_begin) * kThreads + threadIdx.x;
-  if (i >= tk.n_out) return;
-  // the output index's digits: 32-bit, divisions by the legs' invariant
-  // merged and bond dims
-  uint32_t rem = (uint32_t)i;
-  uint32_t voff = 0, vstride = 1, ooff = 0, ostride = 1;
-  for (int k = 0; k < tk.g; ++k) {
-    const uint32_t q = fast_div(rem, tk.div_m[k]);
-    const uint32_t mk = rem - q * tk.div_m[k].d;
+  __shared__ double2 Os[2 * kAbsorbCombos];     // d = 2: the operator's [combo][p]
+  __shared__ uint32_t offs[kAbsorbCombos], oidx[kAbsorbCombos];  // a combo's place in the output and in O (p = 0)
+  const AbsorbTask& tk = tasks[find_task(begins, ntask, blockIdx.x)];
+  const int b = (int)(blockIdx.x - tk.block_begin), d = tk.d, g = tk.g;
+  const int c0 = (b / tk.vblocks) * kAbsorbCombos, nc = (int)min((long long)kAbsorbCombos, tk.ncombo - c0);
+  const uint32_t nops = (uint32_t)(tk.ncombo / d);  // prod r: stride of p in O
+  for (int i = threadIdx.x; i < nc; i += kThreads) {
+    uint32_t o = (uint32_t)(c0 + i), off = 0, stride = 1;
+    const uint32_t pout = o / nops, oi = o - pout * nops;
+    o = oi;
+    for (int k = 0; k < g; ++k) {
+      const uint32_t q = o / (uint32_t)tk.r[k];
+      off += (o - q * (uint32_t)tk.r[k]) * (uint32_t)tk.Dv[k] * stride;
+      o = q;
+      stride *= (uint32_t)(tk.Dv[k] * tk.r[k]);
+    }
+    offs[i] = off + pout * stride;
+    oidx[i] = oi + nops * (uint32_t)d * pout;
+    if (d == 2) {
+      Os[2 * i] = tk.O[oidx[i]];
+      Os[2 * i + 1] = tk.O[oidx[i] + nops];
+    }
+  }
+  __syncthreads();
+  // few v: the rest of the block's threads take other combos
+  const uint32_t nv = (uint32_t)tk.nv, width = min(nv, (uint32_t)kThreads), part = threadIdx.x / width, parts = kThreads / width;
+  const uint32_t v = (uint32_t)(b % tk.vblocks) * kThreads + (threadIdx.x - part * width);
+  if (v >= nv || part >= parts) return;
+  uint32_t rem = v, base = 0, stride = 1;
+  for (int k = 0; k < g; ++k) {
+    const uint32_t q = fast_div(rem, tk.div_v[k]);
+    base += (rem - q * tk.div_v[k].d) * stride;
     rem = q;
-    const uint32_t o = fast_div(mk, tk.div_v[k]);
-    voff += (mk - o * tk.div_v[k].d) * vstride;
-    ooff += o * ostride;
-    vstride *= tk.div_v[k].d;
-    ostride *= (uint32_t)tk.r[k];
+    stride *= (uint32_t)(tk.Dv[k] * tk.r[k]);
   }
-  const uint32_t pout = rem;  // < dout
-  const C* V = static_cast<const C*>(tk.V);
-  double2 acc = make_double2(0.0, 0.0);
-  for (int p = 0; p < tk.d; ++p) {
-    const double2 v = to_d2(V[voff + (size_t)vstride * p]);
-    const double2 o = tk.O[ooff + (size_t)ostride * (p + (size_t)tk.d * pout)];
-    acc = acc + v * o;
+  const C* V = static_cast<const C*>(tk.V) + v;
+  C* out = static_cast<C*>(tk.out) + base;
+  float2* out32 = tk.out32 ? tk.out32 + base : nullptr;
+  if (d == 2) {
+    const double2 v0 = to_d2(V[0]), v1 = to_d2(V[nv]);
+#pragma unroll 4
+    for (int i = (int)part; i < nc; i += (int)parts) {
+      const double2 a = v0 * Os[2 * i] + v1 * Os[2 * i + 1];
+      out[offs[i]] = from_d2<C>(a);
+      if (out32) out32[offs[i]] = make_float2((float)a.x, (float)a.y);
+    }
+    return;
   }
-  static_cast<C*>(tk.out)[i] = from_d2<C>(acc);
+  for (int i = (int)part; i < nc; i += (int)parts) {
+    double2 a = make_double2(0.0, 0.0);
+    for (int p = 0; p < d; ++p) a = a + to_d2(V[(size_t)nv * p]) * tk.O[oidx[i] + (size_t)nops * p];
+    out[offs[i]] = from_d2<C>(a);
+    if (out32) out32[offs[i]] = make_float2((float)a.x, (float)a.y);
+  }
 }
 
 // AbsorbTPO, message part (apply.h:110-128): E'[(e,i),(e',i')] = E[e,e'] d_ii'.

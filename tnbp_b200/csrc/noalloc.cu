@@ -176,7 +176,7 @@ void message_noalloc(const double* site, const int32_t* shape, int32_t rank, int
   }
   launch_gram_f64(d_gram, d_zero, 1, (long long)gt.nchunk * gt.ctiles * gt.ctiles, stream);
   CK(cudaGetLastError());
-  k_msg_finalize<double><<<1, kThreads, 0, stream>>>(d_msg);
+  k_msg_finalize<double><<<1, kFinalizeThreads, 0, stream>>>(d_msg);
   CK(cudaGetLastError());
   note_launch(2);
 }

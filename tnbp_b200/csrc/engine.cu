@@ -1091,15 +1091,17 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
   const bool reduced = !entries.empty() && reduced_sweeps(entries[0].job->prec);
   const bool tc_ok = reduced && tcgen05_enabled();
   {
-    // small sites: one CTA each, every message of the site on chip
+    // small sites: one CTA per message, on chip
     std::vector<SiteTask> sts;
     size_t smem = 0;
+    int degree = 1;
     for (auto& e : entries)
       for (const SiteTask& st : e.job->plan.site[e.parity]) {
         sts.push_back(st);
         smem = std::max(smem, site_sweep_smem_bytes(st.D, st.g, st.d));
+        degree = std::max(degree, st.g);
       }
-    add(SweepLaunch::SITE, sts, {}, (long long)sts.size(), (int)smem);
+    add(SweepLaunch::SITE, sts, {}, degree, (int)smem);
   }
   for (size_t w = 0; w < nw; ++w) {
     {
@@ -1334,8 +1336,8 @@ static int launch_batch_t(const SweepBatch& b, cudaStream_t stream) {
       case SweepLaunch::MSG:
         k_msg_finalize<R, MR><<<L.ntask, kFinalizeThreads, 0, stream>>>(static_cast<const MsgTask*>(tasks));
         break;
-      case SweepLaunch::SITE:  // max_din holds the launch's shared memory bytes
-        k_site_sweep<R, MR><<<L.ntask, kThreads, (size_t)L.max_din, stream>>>(static_cast<const SiteTask*>(tasks));
+      case SweepLaunch::SITE:  // max_din holds the launch's shared memory bytes, nblocks the largest degree
+        k_site_sweep<R, MR><<<dim3((unsigned)L.ntask, (unsigned)L.nblocks), kThreads, (size_t)L.max_din, stream>>>(static_cast<const SiteTask*>(tasks));
         break;
       case SweepLaunch::SUM:
         k_segmented_sum<<<L.ntask, kThreads, 0, stream>>>(static_cast<const SumTask*>(tasks));
@@ -1440,7 +1442,7 @@ bool leg_gram_enabled() {
 }
 
 // Every site whose tensor, two work buffers, messages and Gram partials fit
-// kSiteSmemMax of shared memory is swept whole by one CTA (k_site_sweep);
+// kSiteSmemMax of shared memory is swept on chip, one CTA per message (k_site_sweep);
 // the other sites take the per-level path.  Measured on the random-circuit
 // workload (10x10, BP at D <= 8): BP loops 4.6-5.7 ms per solve against
 // 23-33 ms per-level (mixed), 4.9-6.3 against 8.0-8.5 ms (complex128); the

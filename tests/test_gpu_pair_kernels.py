@@ -43,3 +43,14 @@ def test_degree_four_site_matches_oracle(dims, prec):
             tb.BeliefPropagation(st)
             got = [st.get_message(m) for m in range(8)]
             assert max(float(np.max(np.abs(a - b))) for a, b in zip(got, F)) <= 2e-5
+
+
+# Where a plane's elements run along memory or consecutive planes do, in
+# copies of two elements or (odd extents) of one
+FORMS = [(1, 1, 32, 32), (1, 1, 17, 9), (2, 1, 9, 8), (3, 1, 32, 32), (2, 5, 16, 16), (1, 4, 31, 7), (12, 2, 3, 1), (30, 14, 23, 24)]
+
+
+@pytest.mark.parametrize("prec", [tb.MIXED, tb.C64], ids=["mixed", "c64"])
+@pytest.mark.parametrize("dims", FORMS, ids=["x".join(map(str, d)) for d in FORMS])
+def test_memory_forms_match_oracle(dims, prec):
+    test_degree_four_site_matches_oracle(dims, prec)

@@ -13,14 +13,13 @@
 // tensor 12 times per pair; here 2 reads remain, and the bound moves from
 // HBM and launch tails to shared memory (operand stores and MMA reads, about
 // 6000 cycles per tile at D = 32) and the conversions between hand-overs
-// (12600 to 15100 cycles per tile measured).  One 8x8 sweep at D = 32 (36
-// degree-4 sites): 3.96 ms in the separate kernels, 1.92 ms here; 6x6 at
+// (11900 to 12500 cycles per tile measured).  One 8x8 sweep at D = 32 (36
+// degree-4 sites): 3.96 ms in the separate kernels, 1.60 ms here; 6x6 at
 // D = 16: 0.17 -> 0.10 ms.
 //
 // A tile is P planes (P Dx, P Dy <= 128 rows): raw complex64 planes arrive by
-// cp.async, two tiles in flight, element (o, x, y) at y PE + o Dx + x with PE
-// odd, so that rows (o, x) over y and rows (o, y) over x both read without
-// bank conflicts.  Per target (say x; for y the roles swap):
+// cp.async, two tiles in flight, placed as PairLayout says.  Per target (say
+// x; for y the roles swap):
 //   1. rows (o, x) of W, split hi/lo (3xTF32), go to tensor memory as the A
 //      operand; D1 = A_re [E_re | E_im], D2 = A_im [E_re | E_im] (hi.hi +
 //      hi.lo + lo.hi, A from TMEM, 24 MMAs of N = 64 at D = 32), so only the
@@ -54,20 +53,117 @@ constexpr int kPairThreads = 32 * (kPairWarps + 1 + kPairLoaders);
 constexpr int kPairRegsWork = 112, kPairRegsFeed = 32;
 static_assert(kPairWarps * kPairRegsWork + (1 + kPairLoaders) * kPairRegsFeed <= 96 * (kPairWarps + 1 + kPairLoaders),
               "register split");
-constexpr int kPairRawElems = 32 * 129;                      // one tensor's planes of a tile
+constexpr int kPairRawElems = 32 * 128;                      // one tensor's planes of a tile
 constexpr int kPairWaitLimit = 1 << 22;
 constexpr uint32_t kPairE = 64 * 32 * 4;                     // one of E's operands (N = 64, K = 32)
-constexpr uint32_t kPairOp = 128 * 64 * 4;                   // one Gram operand of a stage (128 rows, 64 columns)
+// One Gram operand of a stage: 128 rows, 16 groups of four columns, these 32
+// or 16 bytes further apart than they are large, so that the planes of one
+// row of PairLayout's second form land in distinct banks.
+__host__ __device__ constexpr uint32_t pair_group(uint32_t P) { return 128 * 16 + (P == 4 ? 32 : 16); }
+constexpr uint32_t kPairOp = 16 * pair_group(4);
 __host__ __device__ constexpr size_t pair_smem_bytes() {
-  return 1024 + 4 * (size_t)kPairE + 2 * (size_t)kPairOp + 4 * (size_t)kPairRawElems * 8 + 128;
+  return 128 + 4 * (size_t)kPairE + 2 * (size_t)kPairOp + 4 * (size_t)kPairRawElems * 8 + 128;
 }
 // Planes per tile: 4 (8 up to dimension 16), so that the padded rows of
 // either target stay within 128 and a Gram stage of 16 (8) of their columns
 // within 64.
 __host__ __device__ inline int pair_planes(int Dx, int Dy) { return (Dx > Dy ? Dx : Dy) <= 16 ? 8 : 4; }
-// Element x of plane o lies at x ^ pair_swizzle(o): loads that run along o
-// then write distinct banks; groups of four stay together.
-__host__ __device__ __forceinline__ uint32_t pair_swizzle(uint32_t o, uint32_t Xp) { return 4u * (o & (Xp % 16 == 0 ? 3u : 1u)); }
+// Where a tile's element (o, x, y) lies: y PE + (e ^ swz(y)), PE = P Xp, with
+// e running as memory does: e = o Xp + x when planes are contiguous (L1 = 1),
+// e = x P + o when consecutive o are.  So 16-byte copies, two elements each,
+// fit both forms when Dx (L1) is even and the tensors are 16-byte aligned;
+// with one form for both, memory that runs along o took 8-byte copies in
+// 32-byte pieces (D = 32: 15100 -> 12500 cycles per tile here, 10700 -> 8000
+// in k_pair_absorb_tc).  A tile's rows are numbered as e, (o, x),
+// or likewise with y for x, (o, y).  The swizzle makes reads of both kinds
+// free of bank conflicts: rows (o, x) read eight bytes at one y, consecutive
+// lanes consecutive e; rows (o, y) read a pair (x, x + 1) in the first form,
+// whose eight lanes differ in y, and eight bytes in the second, whose sixteen
+// lanes are P planes of 16 / P different y.
+template <uint32_t P>
+struct PairLayout {
+  uint32_t along_x, Xp, Yp, PE;  // along_x: the first form
+  __device__ __forceinline__ void set(bool first_form, uint32_t Dx, uint32_t Dy) {
+    along_x = first_form;
+    Xp = (Dx + 7u) & ~7u;
+    Yp = (Dy + 7u) & ~7u;
+    PE = P * Xp;
+  }
+  __device__ __forceinline__ uint32_t swz(uint32_t y) const { return along_x ? 2u * (y & 7u) : P * (y & (16u / P - 1u)); }
+  // (o, i) of row r, i = x or y padded to N
+  __device__ __forceinline__ void row(uint32_t r, uint32_t N, uint32_t& o, uint32_t& i) const {
+    o = along_x ? r / N : r % P;
+    i = along_x ? r - o * N : r / P;
+  }
+};
+// A thread's row of a tile, and reads and writes of its groups of four
+// columns j (j % 2 the same for every one of a thread).
+template <uint32_t P>
+struct PairRow {
+  uint32_t ex, ey, base_y, swz_y, PE;  // ex: swizzled for y = 4 j
+  uint32_t along_x, step_k, mask_k;
+  __device__ __forceinline__ void set(const PairLayout<P>& l, uint32_t row, uint32_t odd) {
+    const uint32_t rx = row < P * l.Xp ? row : 0, ry = row < P * l.Yp ? row : 0;
+    uint32_t o, y;
+    l.row(ry, l.Yp, o, y);
+    along_x = l.along_x;
+    PE = l.PE;
+    ex = rx ^ l.swz(4 * odd);
+    step_k = along_x ? 2 : P;
+    mask_k = along_x ? 3 : 16 / P - 1;
+    base_y = y * PE;
+    ey = along_x ? o * l.Xp : o;
+    swz_y = l.swz(y);
+  }
+  // (o, x) at y = 4 j + k
+  __device__ __forceinline__ uint32_t at_x(uint32_t j, uint32_t k) const {
+    return (ex ^ (step_k * (k & mask_k))) + (4 * j + k) * PE;
+  }
+  // (o, y) at x = 4 j; the three after it are this ^ 1, 2, 3 (^ P, 2 P, 3 P in the second form)
+  template <bool Form>
+  __device__ __forceinline__ uint32_t at_y(uint32_t j) const {
+    return base_y + ((ey + (Form ? 4 : 4 * P) * j) ^ swz_y);
+  }
+  // Form: along_x, known to the caller so that a loop's reads need not wait
+  // for each other's branches
+  template <bool Form>
+  __device__ __forceinline__ void read(const float2* t, bool target_y, uint32_t j, float4& re, float4& im) const {
+    float2 a, b, c, d;
+    if (!target_y) {
+      a = t[at_x(j, 0)];
+      b = t[at_x(j, 1)];
+      c = t[at_x(j, 2)];
+      d = t[at_x(j, 3)];
+    } else if constexpr (Form) {
+      const uint32_t i = at_y<Form>(j);
+      const float4 u = *reinterpret_cast<const float4*>(t + i), v = *reinterpret_cast<const float4*>(t + (i ^ 2));
+      re = make_float4(u.x, u.z, v.x, v.z);
+      im = make_float4(u.y, u.w, v.y, v.w);
+      return;
+    } else {
+      const uint32_t i = at_y<Form>(j);
+      a = t[i];
+      b = t[i ^ P];
+      c = t[i ^ (2 * P)];
+      d = t[i ^ (3 * P)];
+    }
+    re = make_float4(a.x, b.x, c.x, d.x);
+    im = make_float4(a.y, b.y, c.y, d.y);
+  }
+  template <bool Form>
+  __device__ __forceinline__ void write(float2* t, bool target_y, uint32_t j, float4 re, float4 im) const {
+    const uint32_t i = at_y<Form>(j);
+    if (target_y && Form) {
+      *reinterpret_cast<float4*>(t + i) = make_float4(re.x, im.x, re.y, im.y);
+      *reinterpret_cast<float4*>(t + (i ^ 2)) = make_float4(re.z, im.z, re.w, im.w);
+      return;
+    }
+    t[target_y ? i : at_x(j, 0)] = make_float2(re.x, im.x);
+    t[target_y ? i ^ P : at_x(j, 1)] = make_float2(re.y, im.y);
+    t[target_y ? i ^ (2 * P) : at_x(j, 2)] = make_float2(re.z, im.z);
+    t[target_y ? i ^ (3 * P) : at_x(j, 3)] = make_float2(re.w, im.w);
+  }
+};
 
 // The sites that take it: degree 4, every bond dimension at most 32.
 __host__ __device__ inline bool pair_ok(const int* D, int g) {
@@ -163,11 +259,22 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void cp16(float2* dst, const float2* src, bool valid) {
+  const uint32_t d = smem_u32(dst);
+  asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
 __device__ __forceinline__ void cp8(float2* dst, const float2* src, bool valid) {
   const uint32_t d = smem_u32(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
 }
 }  // namespace tc
+
+// Whether two neighbouring elements e of a tile are always 16 aligned bytes
+// of both tensors, and both or neither within them.
+__device__ __forceinline__ bool pair_wide(const LegPairTask& tk) {
+  const int run = tk.L1 == 1 ? tk.Dx : (int)tk.L1;
+  return (run & 1) == 0 && ((reinterpret_cast<uintptr_t>(tk.W) | reinterpret_cast<uintptr_t>(tk.V)) & 15) == 0;
+}
 
 // The messages' operands, E_y then E_x, hi then lo each: element (n, k) of
 // N = 2 Np rows (re, im), K = Np columns; by `nwarp` warps.
@@ -203,7 +310,7 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
                                           long long ntile_all, uint32_t block, uint32_t nblock) {
   using namespace tc;
   extern __shared__ __align__(1024) unsigned char pr_smem_raw[];
-  unsigned char* smem = pr_smem_raw + ((1024 - (smem_u32(pr_smem_raw) & 1023)) & 1023);
+  unsigned char* smem = pr_smem_raw + ((128 - (smem_u32(pr_smem_raw) & 127)) & 127);
   unsigned char* e_op = smem;                       // E_y hi, lo, E_x hi, lo
   unsigned char* g_op = e_op + 4 * kPairE;          // Gram operands of P and of V
   float2* raw = reinterpret_cast<float2*>(g_op + 2 * kPairOp);  // [tile parity][W, V]
@@ -268,8 +375,10 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
     double acc[2][16];
     // of the chunk's task: padded dimensions and groups, this thread's place
     // in a tile and in the operands
-    uint32_t Xp = 0, Yp = 0, PE = 0, gx = 0, gy = 0, ox = 0, xx = 0, oy = 0, yy = 0, base_x = 0, base_y = 0, swz_y = 0, op_x = 0,
-             op_y = 0;
+    uint32_t gx = 0, gy = 0, op_x = 0, op_y = 0;
+    bool in_x = false, in_y = false;  // this thread has a row
+    uint32_t along_x = 1;
+    PairRow<P> pr_row;
 
     auto drain = [&](double (&a)[16], uint32_t col) {
 #pragma unroll
@@ -285,17 +394,9 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
         for (int i = 0; i < 8; ++i) a[8 * h + i] += (double)(v[i] + u[i]);
       }
     };
-    // group j (four columns) of this row: along y for (o, x), along x for (o, y)
-    auto read4 = [&](const float2* t, bool target_y, uint32_t j, float4& re, float4& im) {
-      const uint32_t step = target_y ? 1u : PE;
-      const float2* p = t + (target_y ? base_y + ((4 * j) ^ swz_y) : base_x + 4 * j * PE);
-      const float2 a = p[0], b = p[step], c = p[2 * step], d = p[3 * step];
-      re = make_float4(a.x, b.x, c.x, d.x);
-      im = make_float4(a.y, b.y, c.y, d.y);
-    };
     // rows of W as the A operand in tensor memory: [re_hi | im_hi | re_lo |
     // im_lo] of 32 columns each
-    auto put_a = [&](const float2* w, bool target_y) {
+    auto put_a_form = [&](const float2* w, bool target_y, auto form) {
       const uint32_t n = target_y ? gx : gy;
 #pragma unroll
       for (uint32_t i = 0; i < 2; ++i) {
@@ -303,7 +404,7 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
         if (j < n) {
           float4 re, im, rh, rl, ih, il;
           const uint32_t c = lanes + 4 * j;
-          read4(w, target_y, j, re, im);
+          pr_row.template read<decltype(form)::value>(w, target_y, j, re, im);
           split4(re, rh, rl);
           split4(im, ih, il);
           tmem_st4(c, rh);
@@ -313,6 +414,10 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
         }
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    };
+    auto put_a = [&](const float2* w, bool target_y) {
+      if (!target_y || along_x) put_a_form(w, target_y, std::true_type{});
+      else put_a_form(w, target_y, std::false_type{});
     };
     // P of this row: groups g and g + 4
     float4 pr[2], pi[2];
@@ -369,14 +474,15 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
       const uint32_t first = per * s, count = min(per, n - first);
       const uint32_t jp = per == 4 ? g : g - first, jv = per == 4 ? (g + 2) & 3u : ((g + 2) & 3u) - first;  // within the stage
       if (!fresh && !gram_done()) return false;
-      if ((target_y ? oy : ox) < P) {
+      if (target_y ? in_y : in_x) {
         unsigned char* op = g_op + (target_y ? op_y : op_x);
         if (jv < count) {
           float4 vr, vi;
-          read4(v, target_y, first + jv, vr, vi);
-          put_op(op + kPairOp + jv * (P * 128 * 16), vr, vi);
+          if (!target_y || along_x) pr_row.template read<true>(v, target_y, first + jv, vr, vi);
+          else pr_row.template read<false>(v, target_y, first + jv, vr, vi);
+          put_op(op + kPairOp + jv * (P * pair_group(P)), vr, vi);
         }
-        if (jp < count) put_op(op + jp * (P * 128 * 16), re, im);
+        if (jp < count) put_op(op + jp * (P * pair_group(P)), re, im);
       }
       publish(bar_ready);
       return true;
@@ -391,21 +497,20 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
     const int ntile = min(tk.chunk_tiles, (int)((tk.n_outer + P - 1) / P) - ch.chunk * tk.chunk_tiles);
     if (ch.ti != cur) {  // no MMA is in flight between chunks
       cur = ch.ti;
-      Xp = uniform(((uint32_t)tk.Dx + 7u) & ~7u);
-      Yp = uniform(((uint32_t)tk.Dy + 7u) & ~7u);
-      PE = (P * Xp) | 1u;
-      gx = Xp / 4;
-      gy = Yp / 4;
-      ox = (uint32_t)row / Xp;
-      xx = (uint32_t)row - ox * Xp;
-      oy = (uint32_t)row / Yp;
-      yy = (uint32_t)row - oy * Yp;
-      base_x = ox < P ? ox * Xp + (xx ^ pair_swizzle(ox, Xp)) : 0;  // + y PE
-      base_y = oy < P ? yy * PE + oy * Xp : 0;                      // + (x ^ swz_y)
-      swz_y = pair_swizzle(oy, Xp);
-      op_x = ox * (128 * 16) + (xx >> 3) * 128 + (xx & 7) * 16;  // + P 2048 per group
-      op_y = oy * (128 * 16) + (yy >> 3) * 128 + (yy & 7) * 16;
-      build_pair_e<MR>(tk, e_op, Xp, Yp, warp, lane, kPairWarps);
+      PairLayout<P> lay;
+      lay.set(tk.L1 == 1, (uint32_t)tk.Dx, (uint32_t)tk.Dy);
+      along_x = uniform(lay.along_x);
+      gx = lay.Xp / 4;
+      gy = lay.Yp / 4;
+      in_x = (uint32_t)row < P * lay.Xp;
+      in_y = (uint32_t)row < P * lay.Yp;
+      pr_row.set(lay, (uint32_t)row, g & 1u);
+      uint32_t o, i;
+      lay.row((uint32_t)row, lay.Xp, o, i);
+      op_x = o * pair_group(P) + (i >> 3) * 128 + (i & 7) * 16;  // + P pair_group per group of four columns
+      lay.row((uint32_t)row, lay.Yp, o, i);
+      op_y = o * pair_group(P) + (i >> 3) * 128 + (i & 7) * 16;
+      build_pair_e<MR>(tk, e_op, lay.Xp, lay.Yp, warp, lane, kPairWarps);
     }
 #pragma unroll
     for (int i = 0; i < 16; ++i) acc[0][i] = acc[1][i] = 0.0;
@@ -507,7 +612,7 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
         }
         __syncwarp();
       };
-      const uint64_t da = smem_desc(g0, 128 * 16, 128), db = smem_desc(g0 + kPairOp, 128 * 16, 128);
+      const uint64_t da = smem_desc(g0, pair_group(P), 128), db = smem_desc(g0 + kPairOp, pair_group(P), 128);
       auto stage = [&](uint32_t target, uint32_t count, uint32_t accumulate) {
         ok = wait(bar_ready, gram_ph);
         gram_ph ^= 1u;
@@ -516,7 +621,7 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
         if (elect_one()) {
 #pragma unroll
           for (uint32_t s = 0; s < 8; ++s)
-            if (s < ks) mma_tf32(d, da + 256 * s, db + 256 * s, idesc, accumulate + s);
+            if (s < ks) mma_tf32(d, da + pair_group(P) / 8 * s, db + pair_group(P) / 8 * s, idesc, accumulate + s);
           mma_commit(bar_done);
         }
         __syncwarp();
@@ -537,9 +642,8 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
         }
       }
     } else {
-      // ---- the loading warps: for each y the P Xp elements (o, x) of a row,
-      // 32 at a time, in the order in which memory runs (x when the plane is
-      // contiguous, o when consecutive o are); padding is written as zeros
+      // ---- the loading warps: of each y the elements e of a tile, lanes along
+      // memory, one or two elements per copy; padding is written as zeros
       uint32_t T = 0;
       bool ok = true;
       const uint32_t y0 = (uint32_t)(warp - kPairWarps - 1);
@@ -547,31 +651,45 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
         const LegPairTask& tk = tasks[ch.ti];
         const int ntile = min(tk.chunk_tiles, (int)((tk.n_outer + P - 1) / P) - ch.chunk * tk.chunk_tiles);
         const uint32_t Dx = (uint32_t)tk.Dx, Dy = (uint32_t)tk.Dy, L1 = (uint32_t)tk.L1, O = (uint32_t)tk.n_outer;
-        const uint32_t Xp = (Dx + 7u) & ~7u, Yp = (Dy + 7u) & ~7u, PE = (P * Xp) | 1u;
+        PairLayout<P> lay;
+        lay.set(L1 == 1, Dx, Dy);
         const float2* __restrict__ Wg = static_cast<const float2*>(tk.W);
         const ptrdiff_t VmW = static_cast<const float2*>(tk.V) - Wg;
+        auto copy = [&](auto width, float2* dst, uint32_t o0) {
+          constexpr uint32_t w = decltype(width)::value;
+#pragma unroll 1
+          for (uint32_t e = w * (uint32_t)lane; e < lay.PE; e += 32 * w) {
+            uint32_t o, x;
+            lay.row(e, lay.Xp, o, x);
+            const uint32_t oo = o0 + o, hi = fast_div(oo, tk.div_l), lo = oo - hi * L1;
+            const bool ok_ox = oo < O && x < Dx;
+            const float2* p = Wg + (ok_ox ? (size_t)lo + (size_t)L1 * (x + Dx * (y0 + Dy * (size_t)hi)) : 0);
+            const size_t dy = ok_ox ? (size_t)kPairLoaders * L1 * Dx : 0;
+            float2* d = dst + y0 * lay.PE;
+#pragma unroll 2
+            for (uint32_t y = y0; y < lay.Yp; y += kPairLoaders) {
+              const bool in = ok_ox && y < Dy;
+              float2* de = d + (e ^ lay.swz(y));
+              if constexpr (w == 2) {
+                cp16(de, in ? p : Wg, in);
+                cp16(de + kPairRawElems, in ? p + VmW : Wg, in);
+              } else {
+                cp8(de, in ? p : Wg, in);
+                cp8(de + kPairRawElems, in ? p + VmW : Wg, in);
+              }
+              p += dy;
+              d += kPairLoaders * lay.PE;
+            }
+          }
+        };
+        const bool wide = pair_wide(tk);
         for (int t = 0; t < ntile && ok; ++t, ++T) {
           const uint32_t st = T & 1u;
           if (T >= 2 && !(ok = wait(bar_free + 8u * st, ((T >> 1) - 1) & 1u))) break;
           float2* dst = raw + (size_t)st * 2 * kPairRawElems;
           const uint32_t o0 = (uint32_t)(ch.chunk * tk.chunk_tiles + t) * P;
-#pragma unroll 1
-          for (uint32_t el = (uint32_t)lane; el < P * Xp; el += 32) {
-            const uint32_t o = L1 == 1 ? el / Xp : el % P, x = L1 == 1 ? el - o * Xp : el / P;
-            const uint32_t oo = o0 + o, hi = fast_div(oo, tk.div_l), lo = oo - hi * L1;
-            const bool ok_ox = oo < O && x < Dx;
-            const float2* w = Wg + (ok_ox ? (size_t)lo + (size_t)L1 * (x + Dx * (y0 + Dy * (size_t)hi)) : 0);
-            const size_t dy = ok_ox ? (size_t)kPairLoaders * L1 * Dx : 0;
-            float2* d = dst + y0 * PE + o * Xp + (x ^ pair_swizzle(o, Xp));
-#pragma unroll 2
-            for (uint32_t y = y0; y < Yp; y += kPairLoaders) {
-              const bool in = ok_ox && y < Dy;
-              cp8(d, in ? w : Wg, in);
-              cp8(d + kPairRawElems, in ? w + VmW : Wg, in);
-              w += dy;
-              d += kPairLoaders * PE;
-            }
-          }
+          if (wide) copy(std::integral_constant<uint32_t, 2>{}, dst, o0);
+          else copy(std::integral_constant<uint32_t, 1>{}, dst, o0);
           // this thread's arrival, when its copies have landed
           asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar_full + 8u * st) : "memory");
         }
@@ -605,14 +723,14 @@ __global__ void __launch_bounds__(tc::kPairThreads, 1)
 // Why: two launches of the leg kernel read and wrote the tensor twice; here it
 // is read and written once, which leaves HBM (64 KB per tile at D = 32, about
 // 2800 cycles per SM) and the two products' MMAs (1700 cycles) as bounds.
-// One 8x8 sweep at D = 32: 1.86 ms in the leg kernel, 1.15 ms here (6000
-// cycles per tile when planes are contiguous, 10700 when memory runs along o
+// One 8x8 sweep at D = 32: 1.86 ms in the leg kernel, 0.88 ms here (5400
+// cycles per tile when planes are contiguous, 8000 when memory runs along o
 // and a tile is 32-byte pieces); 6x6 at D = 16: 0.09 -> 0.04 ms.
 //
 // Tiles, rows and tensor-memory operands are those of pair_gram.  The first
 // product's rows (o, x) go back over the tile they came from, the second
 // takes rows (o, y) from there, and its rows return to the same place, from
-// which the tile is written out as memory runs.  256 threads, two CTAs per SM
+// which the tile is written out as memory runs.  512 threads, two CTAs per SM
 // (98 KB of shared memory, 256 tensor-memory columns each): one converts
 // while the other waits.
 // ---------------------------------------------------------------------------
@@ -620,7 +738,7 @@ namespace tc {
 constexpr int kAbsorbThreads = 512;
 constexpr uint32_t kAbsorbG = kAbsorbThreads / 128;  // warps that share a row
 __host__ __device__ constexpr size_t absorb_smem_bytes() {
-  return 1024 + 4 * (size_t)kPairE + 2 * (size_t)kPairRawElems * 8 + 64;
+  return 128 + 4 * (size_t)kPairE + 2 * (size_t)kPairRawElems * 8 + 64;
 }
 }  // namespace tc
 
@@ -629,7 +747,7 @@ __device__ __forceinline__ void pair_absorb(const LegPairTask* __restrict__ task
                                             long long ntile_all, uint32_t block, uint32_t nblock) {
   using namespace tc;
   extern __shared__ __align__(1024) unsigned char pr_smem_raw[];
-  unsigned char* e_op = pr_smem_raw + ((1024 - (smem_u32(pr_smem_raw) & 1023)) & 1023);  // E_y hi, lo, E_x hi, lo
+  unsigned char* e_op = pr_smem_raw + ((128 - (smem_u32(pr_smem_raw) & 127)) & 127);  // E_y hi, lo, E_x hi, lo
   float2* raw = reinterpret_cast<float2*>(e_op + 4 * kPairE);                             // two tiles
   uint64_t* bar = reinterpret_cast<uint64_t*>(raw + 2 * kPairRawElems);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
@@ -656,18 +774,22 @@ __device__ __forceinline__ void pair_absorb(const LegPairTask* __restrict__ task
   // has those with j % 4 == g
   const int row = 32 * (warp & 3) + lane;
   const uint32_t g = (uint32_t)warp >> 2, lanes = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-  // of the task: padded dimensions, this thread's place in a tile
-  uint32_t Xp = 8, Yp = 8, PE = 0, base_x = 0, base_y = 0, swz_y = 0;
-  // and its copies: the element (o, x) of every y = g + 4 k, at cp_d + y PE of
-  // a tile and at cp_off + y cp_step (cp_plane per unit of o / L1) in memory
-  uint32_t cp_o = 0, cp_d = 0, L1 = 1, Dy = 0, n_outer = 0;
-  bool cp_mine = false, cp_pad = false;
+  // of the task: its layout, this thread's row
+  PairLayout<P> lay{1, 8, 8, 8 * P};
+  PairRow<P> my;
+  my.set(lay, 0, 0);
+  bool in_x = false, in_y = false;
+  // and its copies: two elements of every eighth y from cp_y on or one of
+  // every fourth, from cp_d of a tile (four y's flip the swizzle by cp_flip)
+  // and cp_off in memory, there cp_step apart (cp_plane per unit of o / L1)
+  uint32_t cp_o = 0, cp_d = 0, cp_y = 0, cp_flip = 0, L1 = 1, Dy = 0, n_outer = 0;
+  bool cp_mine = false, cp_pad = false, wide = false;
   size_t cp_off = 0, cp_step = 0, cp_plane = 0;
   FastDiv div_l{1, 1, 0};
   const float2* src = nullptr;
   ptrdiff_t dst = 0;  // output minus input
 
-  // offset at y = g of this thread's element in tile lt; false if it has none
+  // offset at y = cp_y of this thread's element in tile lt; false if it has none
   auto place = [&](uint32_t lt, size_t& off) {
     const uint32_t oo = lt * P + cp_o, hi = fast_div(oo, div_l);
     off = cp_off + (oo - hi * L1) + cp_plane * hi;
@@ -678,29 +800,39 @@ __device__ __forceinline__ void pair_absorb(const LegPairTask* __restrict__ task
       size_t off;
       const bool ok = place(lt, off);
       const float2* p = ok ? src + off : src;
-      float2* d = raw + (size_t)stage * kPairRawElems + cp_d;
+      float2* t = raw + (size_t)stage * kPairRawElems;
+      uint32_t d = cp_d;
+      if (wide) {
 #pragma unroll 4
-      for (uint32_t y = g; y < Yp; y += kAbsorbG) {
-        const bool in = ok && y < Dy;
-        cp8(d, in ? p : src, in);
-        p += cp_step;
-        d += kAbsorbG * PE;
+        for (uint32_t y = cp_y; y < lay.Yp; y += kAbsorbThreads / 64) {
+          const bool in = ok && y < Dy;
+          cp16(t + d, in ? p : src, in);
+          p += cp_step;
+          d += kAbsorbThreads / 64 * lay.PE;
+        }
+      } else {
+#pragma unroll 4
+        for (uint32_t y = cp_y; y < lay.Yp; y += kAbsorbG) {
+          const bool in = ok && y < Dy;
+          cp8(t + d, in ? p : src, in);
+          p += cp_step;
+          d = (d ^ cp_flip) + kAbsorbG * lay.PE;
+        }
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   // rows of the tile as the A operand: [re_hi | im_hi | re_lo | im_lo]
-  auto put_a = [&](const float2* t, bool target_y) {
-    const uint32_t n = (target_y ? Xp : Yp) / 4;
+  auto put_a_form = [&](const float2* t, bool target_y, auto form) {
+    const uint32_t n = (target_y ? lay.Xp : lay.Yp) / 4;
 #pragma unroll
     for (uint32_t j = g; j < 8; j += kAbsorbG)
       if (j < n) {
-        const uint32_t step = target_y ? 1u : PE, c = lanes + 4 * j;
-        const float2* p = t + (target_y ? base_y + ((4 * j) ^ swz_y) : base_x + 4 * j * PE);
-        const float2 e0 = p[0], e1 = p[step], e2 = p[2 * step], e3 = p[3 * step];
-        float4 rh, rl, ih, il;
-        split4(make_float4(e0.x, e1.x, e2.x, e3.x), rh, rl);
-        split4(make_float4(e0.y, e1.y, e2.y, e3.y), ih, il);
+        const uint32_t c = lanes + 4 * j;
+        float4 re, im, rh, rl, ih, il;
+        my.template read<decltype(form)::value>(t, target_y, j, re, im);
+        split4(re, rh, rl);
+        split4(im, ih, il);
         tmem_st4(c, rh);
         tmem_st4(c + 32u, ih);
         tmem_st4(c + 64u, rl);
@@ -709,28 +841,34 @@ __device__ __forceinline__ void pair_absorb(const LegPairTask* __restrict__ task
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
   };
   // the product's rows back over the tile
-  auto put_back = [&](float2* t, bool target_y) {
-    const uint32_t Np = target_y ? Xp : Yp, n = Np / 4;
-    const bool valid = (uint32_t)row < P * (target_y ? Yp : Xp);
+  auto put_back_form = [&](float2* t, bool target_y, auto form) {
+    const uint32_t Np = target_y ? lay.Xp : lay.Yp, n = Np / 4;
+    const bool valid = target_y ? in_y : in_x;
 #pragma unroll
     for (uint32_t j = g; j < 8; j += kAbsorbG)
       if (j < n) {
-        const uint32_t step = target_y ? 1u : PE, c = lanes + kColP + 4 * j;
+        const uint32_t c = lanes + kColP + 4 * j;
         float rr[4], ri[4], ir[4], ii[4];
         tmem_ld4_async(c, rr);            // A_re E_re
         tmem_ld4_async(c + Np, ri);       // A_re E_im
         tmem_ld4_async(c + 64, ir);       // A_im E_re
         tmem_ld4_async(c + 64 + Np, ii);  // A_im E_im
         tmem_ld_wait16(rr, ri, ir, ii);
-        if (valid) {
-          float2* p = t + (target_y ? base_y + ((4 * j) ^ swz_y) : base_x + 4 * j * PE);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) p[k * step] = make_float2(rr[k] - ii[k], ri[k] + ir[k]);
-        }
+        if (valid)
+          my.template write<decltype(form)::value>(t, target_y, j, make_float4(rr[0] - ii[0], rr[1] - ii[1], rr[2] - ii[2], rr[3] - ii[3]),
+                   make_float4(ri[0] + ir[0], ri[1] + ir[1], ri[2] + ir[2], ri[3] + ir[3]));
       }
   };
+  auto put_a = [&](const float2* t, bool target_y) {
+    if (!target_y || lay.along_x) put_a_form(t, target_y, std::true_type{});
+    else put_a_form(t, target_y, std::false_type{});
+  };
+  auto put_back = [&](float2* t, bool target_y) {
+    if (!target_y || lay.along_x) put_back_form(t, target_y, std::true_type{});
+    else put_back_form(t, target_y, std::false_type{});
+  };
   auto leg_mma = [&](uint32_t which) {  // by warp 0; 0: E_y (K = Yp), 1: E_x
-    const uint32_t k8 = uniform(which ? Xp : Yp) / 8, N2 = 16 * k8, idesc = idesc_tf32(128, 0) | ((N2 >> 3) << 17);
+    const uint32_t k8 = uniform(which ? lay.Xp : lay.Yp) / 8, N2 = 16 * k8, idesc = idesc_tf32(128, 0) | ((N2 >> 3) << 17);
     const uint32_t op = uniform(smem_u32(e_op)) + which * 2 * kPairE;
     const uint64_t dh0 = smem_desc(op, N2 * 16, 128), dl0 = smem_desc(op + kPairE, N2 * 16, 128);
     if (elect_one()) {
@@ -780,27 +918,27 @@ __device__ __forceinline__ void pair_absorb(const LegPairTask* __restrict__ task
       div_l = tk.div_l;
       task_end = begins[ti] + (n_outer + P - 1) / P;
       lt = (uint32_t)(tile - begins[ti]);
-      Xp = (Dx + 7u) & ~7u;
-      Yp = (Dy + 7u) & ~7u;
-      PE = (P * Xp) | 1u;
-      const uint32_t ox = (uint32_t)row / Xp, xx = (uint32_t)row - ox * Xp, oy = (uint32_t)row / Yp, yy = (uint32_t)row - oy * Yp;
-      base_x = ox < P ? ox * Xp + (xx ^ pair_swizzle(ox, Xp)) : 0;  // + y PE
-      base_y = oy < P ? yy * PE + oy * Xp : 0;                      // + (x ^ swz_y)
-      swz_y = pair_swizzle(oy, Xp);
-      // 32 elements (o, x) per instruction as memory runs: along x when the
-      // plane is contiguous, along o when consecutive o are
-      const uint32_t el = (uint32_t)row, o = L1 == 1 ? el / Xp : el % P, x = L1 == 1 ? el - o * Xp : el / P;
-      cp_o = o;
-      cp_mine = o < P && x < Dx;
-      cp_pad = o < P && x < Xp && !cp_mine;
-      cp_d = o * Xp + (x ^ pair_swizzle(o, Xp)) + g * PE;
-      cp_off = (size_t)L1 * (x + (size_t)Dx * g);
-      cp_step = (size_t)L1 * Dx * kAbsorbG;
+      lay.set(L1 == 1, Dx, Dy);
+      lay.along_x = uniform(lay.along_x);
+      my.set(lay, (uint32_t)row, g & 1u);
+      in_x = (uint32_t)row < P * lay.Xp;
+      in_y = (uint32_t)row < P * lay.Yp;
+      wide = pair_wide(tk);
+      const uint32_t e = wide ? 2 * ((uint32_t)tid & 63u) : (uint32_t)row;
+      uint32_t x;
+      lay.row(e, lay.Xp, cp_o, x);
+      cp_y = wide ? (uint32_t)tid >> 6 : g;
+      cp_d = (e ^ lay.swz(cp_y)) + cp_y * lay.PE;
+      cp_flip = lay.swz(4);
+      cp_mine = e < lay.PE && x < Dx;
+      cp_pad = e < lay.PE && !cp_mine;
+      cp_off = (size_t)L1 * (x + (size_t)Dx * cp_y);
+      cp_step = (size_t)L1 * Dx * (wide ? kAbsorbThreads / 64 : kAbsorbG);
       cp_plane = (size_t)L1 * Dx * Dy;
       src = static_cast<const float2*>(tk.V);
       dst = static_cast<const float2*>(tk.W) - src;
       loaded = false;
-      build_pair_e<MR>(tk, e_op, Xp, Yp, warp, lane, kAbsorbThreads / 32);
+      build_pair_e<MR>(tk, e_op, lay.Xp, lay.Yp, warp, lane, kAbsorbThreads / 32);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (!loaded) {
@@ -826,12 +964,21 @@ __device__ __forceinline__ void pair_absorb(const LegPairTask* __restrict__ task
     size_t off;
     if (place(lt, off)) {
       float2* out = const_cast<float2*>(src) + dst + off;
-      const float2* s = t + cp_d;
+      uint32_t d = cp_d;
+      if (wide) {
 #pragma unroll 4
-      for (uint32_t y = g; y < Dy; y += kAbsorbG) {
-        *out = *s;
-        out += cp_step;
-        s += kAbsorbG * PE;
+        for (uint32_t y = cp_y; y < Dy; y += kAbsorbThreads / 64) {
+          *reinterpret_cast<float4*>(out) = *reinterpret_cast<const float4*>(t + d);
+          out += cp_step;
+          d += kAbsorbThreads / 64 * lay.PE;
+        }
+      } else {
+#pragma unroll 4
+        for (uint32_t y = cp_y; y < Dy; y += kAbsorbG) {
+          *out = t[d];
+          out += cp_step;
+          d = (d ^ cp_flip) + kAbsorbG * lay.PE;
+        }
       }
     }
   }

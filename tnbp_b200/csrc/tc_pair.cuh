@@ -11,11 +11,14 @@
 //
 // Why: level by level, these two absorptions and Grams read and write a site
 // tensor 12 times per pair; here 2 reads remain, and the bound moves from
-// HBM and launch tails to shared memory (operand stores and MMA reads, about
-// 6000 cycles per tile at D = 32) and the conversions between hand-overs
-// (11900 to 12500 cycles per tile measured).  One 8x8 sweep at D = 32 (36
-// degree-4 sites): 3.96 ms in the separate kernels, 1.60 ms here; 6x6 at
-// D = 16: 0.17 -> 0.10 ms.
+// HBM and launch tails to what lies between the hand-overs of a tile: shared
+// memory (operand stores and MMA reads, about 6000 cycles per tile at D =
+// 32), conversions, FP64 additions and waits.  So two groups of warps, one
+// per target, share the tiles but nothing else and fill each other's gaps
+// (cycles per tile with one group that took the targets in turn: 12200 at D =
+// 32, 9850 at 24, 10600 at 16; now 11550, 8950, 8900).  One 8x8 sweep at
+// D = 32 (36 degree-4 sites): 3.96 ms in the separate kernels, 1.52 ms here;
+// 6x6 at D = 16: 0.17 -> 0.09 ms.
 //
 // A tile is P planes (P Dx, P Dy <= 128 rows): raw complex64 planes arrive by
 // cp.async, two tiles in flight, placed as PairLayout says.  Per target (say
@@ -25,10 +28,10 @@
 //      hi.lo + lo.hi, A from TMEM, 24 MMAs of N = 64 at D = 32), so only the
 //      two 64-column halves of E are kept in shared memory;
 //      P_re = D1_re - D2_im, P_im = D1_im + D2_re
-//   2. P and the matching rows of V become the Gram's operands, half of the y
-//      range at a time: rows [re_hi; im_hi; re_lo; im_lo] x 32 of up to 64
-//      contraction columns (o, y); one M = 128, N = 128 MMA per 8 columns
-//      gives all four hi/lo products
+//   2. P and the matching rows of V become the Gram's operands, eight columns
+//      y at a time: rows [re_hi; im_hi; re_lo; im_lo] x 32 of 8 P contraction
+//      columns (o, y); one M = 128, N = 128 MMA per 8 columns gives all four
+//      hi/lo products
 //   3. the tile's FP32 Gram is added to FP64 registers.
 // A chunk of tiles ends in one FP64 partial per target, reduced by
 // k_msg_finalize in a fixed order.
@@ -46,34 +49,37 @@ namespace tnbp {
 
 namespace tc {
 constexpr int kPairWarps = 16;                               // converting warps
-constexpr int kPairLoaders = 3;                              // loading warps, beside one that issues the MMAs
-constexpr int kPairThreads = 32 * (kPairWarps + 1 + kPairLoaders);
+constexpr int kPairGroup = kPairWarps / 2;                   // those of one target
+constexpr int kPairLoaders = 2;                              // loading warps, beside two that issue the MMAs
+constexpr int kPairThreads = 32 * (kPairWarps + 2 + kPairLoaders);
 // Registers per thread after the split: 512 x 112 + 128 x 32 = 640 x 96, what
 // the launch gives the CTA (64 of the 112 are the FP64 sums).
 constexpr int kPairRegsWork = 112, kPairRegsFeed = 32;
-static_assert(kPairWarps * kPairRegsWork + (1 + kPairLoaders) * kPairRegsFeed <= 96 * (kPairWarps + 1 + kPairLoaders),
+static_assert(kPairWarps * kPairRegsWork + (2 + kPairLoaders) * kPairRegsFeed <= 96 * (kPairWarps + 2 + kPairLoaders),
               "register split");
 constexpr int kPairRawElems = 32 * 128;                      // one tensor's planes of a tile
 constexpr int kPairWaitLimit = 1 << 22;
 constexpr uint32_t kPairE = 64 * 32 * 4;                     // one of E's operands (N = 64, K = 32)
-// One Gram operand of a stage: 128 rows, 16 groups of four columns, these 32
+// One Gram operand of a stage: 128 rows, 2 P groups of four columns, these 32
 // or 16 bytes further apart than they are large, so that the planes of one
 // row of PairLayout's second form land in distinct banks.
 __host__ __device__ constexpr uint32_t pair_group(uint32_t P) { return 128 * 16 + (P == 4 ? 32 : 16); }
-constexpr uint32_t kPairOp = 16 * pair_group(4);
+__host__ __device__ constexpr uint32_t pair_op(uint32_t P) { return 2 * P * pair_group(P); }
+// One tensor's planes of a tile: 32 x 32 x 4 or 16 x 16 x 8
+__host__ __device__ constexpr uint32_t pair_raw(uint32_t P) { return P == 4 ? 32 * 128 : 16 * 128; }
+__host__ __device__ constexpr size_t pair_ring(uint32_t P) { return 4 * ((size_t)pair_op(P) + pair_raw(P) * 8); }
 __host__ __device__ constexpr size_t pair_smem_bytes() {
-  return 128 + 4 * (size_t)kPairE + 2 * (size_t)kPairOp + 4 * (size_t)kPairRawElems * 8 + 128;
+  return 128 + 4 * (size_t)kPairE + (pair_ring(4) > pair_ring(8) ? pair_ring(4) : pair_ring(8)) + 128;
 }
-// Planes per tile: 4 (8 up to dimension 16), so that the padded rows of
-// either target stay within 128 and a Gram stage of 16 (8) of their columns
-// within 64.
+// Planes per tile: 4 (8 up to dimension 16): the padded rows of
+// either target stay within 128.
 __host__ __device__ inline int pair_planes(int Dx, int Dy) { return (Dx > Dy ? Dx : Dy) <= 16 ? 8 : 4; }
 // Where a tile's element (o, x, y) lies: y PE + (e ^ swz(y)), PE = P Xp, with
 // e running as memory does: e = o Xp + x when planes are contiguous (L1 = 1),
 // e = x P + o when consecutive o are.  So 16-byte copies, two elements each,
 // fit both forms when Dx (L1) is even and the tensors are 16-byte aligned;
 // with one form for both, memory that runs along o took 8-byte copies in
-// 32-byte pieces (D = 32: 15100 -> 12500 cycles per tile here, 10700 -> 8000
+// 32-byte pieces (D = 32: 15100 -> 12500 cycles per tile in pair_gram, 10700 -> 8000
 // in k_pair_absorb_tc).  A tile's rows are numbered as e, (o, x),
 // or likewise with y for x, (o, y).  The swizzle makes reads of both kinds
 // free of bank conflicts: rows (o, x) read eight bytes at one y, consecutive
@@ -277,12 +283,12 @@ __device__ __forceinline__ bool pair_wide(const LegPairTask& tk) {
 }
 
 // The messages' operands, E_y then E_x, hi then lo each: element (n, k) of
-// N = 2 Np rows (re, im), K = Np columns; by `nwarp` warps.
+// N = 2 Np rows (re, im), K = Np columns; legs leg0 .. leg1 - 1, by `nwarp` warps.
 template <typename MR>
-__device__ __forceinline__ void build_pair_e(const LegPairTask& tk, unsigned char* e_op, uint32_t Xp, uint32_t Yp, int warp, int lane,
-                                             int nwarp) {
+__device__ __forceinline__ void build_pair_e(const LegPairTask& tk, unsigned char* e_op, uint32_t Xp, uint32_t Yp, int leg0, int leg1,
+                                             int warp, int lane, int nwarp) {
   using namespace tc;
-  for (int leg = 0; leg < 2; ++leg) {
+  for (int leg = leg0; leg < leg1; ++leg) {
     const int D = leg == 0 ? tk.Dy : tk.Dx, Np = leg == 0 ? (int)Yp : (int)Xp, N2 = 2 * Np;
     const typename cvec<MR>::type* E = static_cast<const typename cvec<MR>::type*>(leg == 0 ? tk.Ey : tk.Ex);
     unsigned char* hi_op = e_op + (size_t)leg * 2 * kPairE;
@@ -312,14 +318,15 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
   extern __shared__ __align__(1024) unsigned char pr_smem_raw[];
   unsigned char* smem = pr_smem_raw + ((128 - (smem_u32(pr_smem_raw) & 127)) & 127);
   unsigned char* e_op = smem;                       // E_y hi, lo, E_x hi, lo
-  unsigned char* g_op = e_op + 4 * kPairE;          // Gram operands of P and of V
-  float2* raw = reinterpret_cast<float2*>(g_op + 2 * kPairOp);  // [tile parity][W, V]
-  // mbarriers: leg operands ready, done; Gram operands ready, done; per tile
-  // parity: tile arrived, used
-  uint64_t* bars = reinterpret_cast<uint64_t*>(raw + 4 * kPairRawElems);
-  const uint32_t bar_leg = smem_u32(bars), bar_leg_done = bar_leg + 8, bar_ready = bar_leg + 16, bar_done = bar_leg + 24,
-                 bar_full = bar_leg + 32, bar_free = bar_leg + 48;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  unsigned char* g_op = e_op + 4 * kPairE;          // per target: Gram operands of P and of V
+  constexpr uint32_t kOp = pair_op(P), kRaw = pair_raw(P);
+  float2* raw = reinterpret_cast<float2*>(g_op + 4 * kOp);  // [tile parity][W, V]
+  // mbarriers, per target: leg operands ready, done; Gram operands ready,
+  // done; per tile parity: tile arrived, used; per target: its warps met
+  uint64_t* bars = reinterpret_cast<uint64_t*>(raw + 4 * kRaw);
+  const uint32_t bar_leg = smem_u32(bars), bar_leg_done = bar_leg + 16, bar_ready = bar_leg + 32, bar_done = bar_leg + 48,
+                 bar_full = bar_leg + 64, bar_free = bar_leg + 80, bar_group = bar_leg + 96;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
   volatile int* fail = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 
@@ -327,9 +334,6 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
   const long long share = (ntile_all + nblock - 1) / nblock, first_tile = block * share;
   const long long last_tile = min(ntile_all, first_tile + share);
   if (first_tile >= last_tile) return;
-  // groups of four columns in a row; a Gram stage holds up to `per` of them,
-  // of every plane: one or two stages per target
-  constexpr uint32_t per = P == 4 ? 4u : 2u;
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -337,8 +341,9 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    for (int i = 0; i < 8; ++i) {
-      const uint32_t count = i == 1 || i == 3 ? 1u : i == 4 || i == 5 ? 32u * kPairLoaders : (uint32_t)kPairWarps;
+    for (int i = 0; i < 14; ++i) {
+      const int k = i / 2;  // as listed above
+      const uint32_t count = k == 1 || k == 3 ? 1u : k == 4 ? 32u * kPairLoaders : k == 5 ? (uint32_t)kPairWarps : (uint32_t)kPairGroup;
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bars + i)), "r"(count));
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -348,7 +353,12 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  constexpr uint32_t kColP = 128, kColN = 256;  // A operand at 0, D1 at 128, D2 at 192, N_x at 256, N_y at 384
+  // Tensor memory per target: A's four blocks of kBlk columns at 0, D1 and D2
+  // (2 kBlk each) after them, N's 128 columns over A when its MMAs are done
+  // (four planes: no room) or after D (eight: the next tile's A and its MMAs
+  // do not wait for this tile's N).
+  constexpr uint32_t kBlk = P == 4 ? 32 : 16, kColP = 4 * kBlk, kColN = P == 4 ? 0 : 8 * kBlk;
+  constexpr bool kAhead = P != 4;
 
   // A bounded wait by a whole warp; false (for the whole warp) when it or
   // any other thread of the CTA gave up.
@@ -367,75 +377,77 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
   // leads from the smaller share into the converting warps' code.
   if (warp < kPairWarps) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPairRegsWork));
-    // this thread's row of a tile, (o, x) or (o, y); of its groups of four
-    // columns, j, warps 4 g .. 4 g + 3 hold those with j % 4 == g
-    const int row = 32 * (warp & 3) + lane;
-    const uint32_t g = (uint32_t)warp >> 2;
-    const uint32_t lanes = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-    double acc[2][16];
-    // of the chunk's task: padded dimensions and groups, this thread's place
-    // in a tile and in the operands
-    uint32_t gx = 0, gy = 0, op_x = 0, op_y = 0;
-    bool in_x = false, in_y = false;  // this thread has a row
-    uint32_t along_x = 1;
+    // two groups of warps, one per target, each at its own pace; this
+    // thread's row of a tile, (o, x) for target x, (o, y) for y; of its
+    // groups of four columns, j, those with j % 2 == g
+    const uint32_t target = (uint32_t)warp / kPairGroup, w8 = (uint32_t)warp % kPairGroup;
+    const int row = 32 * (int)(w8 & 3) + lane;
+    const uint32_t g = w8 >> 2;
+    const uint32_t lanes = tmem + 256u * target + ((uint32_t)(32 * (w8 & 3)) << 16);
+    unsigned char* const ops = g_op + target * 2 * kOp;
+    double acc[32];
+    // of the chunk's task: groups in a row, this thread's place in a tile and
+    // in the operands
+    uint32_t n = 0, op_row = 0, along_x = 1;
+    bool in = false;  // this thread has a row
     PairRow<P> pr_row;
 
-    auto drain = [&](double (&a)[16], uint32_t col) {
+    // N of this row: columns 8 i + 4 g + k (those whose place this warp's
+    // part of the next A takes)
+    auto drain = [&]() {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
+      for (int h = 0; h < 4; ++h) {
         float v[8], u[8];
-        const uint32_t c = lanes + col + 16u * g + 8u * h;
+        const uint32_t c = lanes + kColN + 4u * g + 16u * h;
         tmem_ld4_async(c, v);
-        tmem_ld4_async(c + 4, v + 4);
+        tmem_ld4_async(c + 8, v + 4);
         tmem_ld4_async(c + 64, u);
-        tmem_ld4_async(c + 68, u + 4);
+        tmem_ld4_async(c + 72, u + 4);
         tmem_ld_wait16(v, v + 4, u, u + 4);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) a[8 * h + i] += (double)(v[i] + u[i]);
+        for (int i = 0; i < 8; ++i) acc[8 * h + i] += (double)(v[i] + u[i]);
       }
     };
+    auto read4 = [&](const float2* t, uint32_t j, float4& re, float4& im) {
+      if (target == 0 || along_x) pr_row.template read<true>(t, target != 0, j, re, im);
+      else pr_row.template read<false>(t, true, j, re, im);
+    };
     // rows of W as the A operand in tensor memory: [re_hi | im_hi | re_lo |
-    // im_lo] of 32 columns each
-    auto put_a_form = [&](const float2* w, bool target_y, auto form) {
-      const uint32_t n = target_y ? gx : gy;
+    // im_lo] of kBlk columns each
+    auto put_a_form = [&](const float2* w, auto target_y, auto form) {
 #pragma unroll
-      for (uint32_t i = 0; i < 2; ++i) {
-        const uint32_t j = g + 4 * i;
+      for (uint32_t i = 0; i < kBlk / 8; ++i) {
+        const uint32_t j = g + 2 * i;
         if (j < n) {
           float4 re, im, rh, rl, ih, il;
           const uint32_t c = lanes + 4 * j;
-          pr_row.template read<decltype(form)::value>(w, target_y, j, re, im);
+          pr_row.template read<decltype(form)::value>(w, decltype(target_y)::value, j, re, im);
           split4(re, rh, rl);
           split4(im, ih, il);
           tmem_st4(c, rh);
-          tmem_st4(c + 32u, ih);
-          tmem_st4(c + 64u, rl);
-          tmem_st4(c + 96u, il);
+          tmem_st4(c + kBlk, ih);
+          tmem_st4(c + 2 * kBlk, rl);
+          tmem_st4(c + 3 * kBlk, il);
         }
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     };
-    auto put_a = [&](const float2* w, bool target_y) {
-      if (!target_y || along_x) put_a_form(w, target_y, std::true_type{});
-      else put_a_form(w, target_y, std::false_type{});
+    auto put_a = [&](const float2* w) {
+      if (target == 0) put_a_form(w, std::false_type{}, std::true_type{});
+      else if (along_x) put_a_form(w, std::true_type{}, std::true_type{});
+      else put_a_form(w, std::true_type{}, std::false_type{});
     };
-    // P of this row: groups g and g + 4
-    float4 pr[2], pi[2];
-    auto get_p = [&](uint32_t n) {
-      const uint32_t Np = 4 * n, c0 = lanes + kColP + 4 * g;
-#pragma unroll
-      for (uint32_t i = 0; i < 2; ++i)
-        if (g + 4 * i < n) {
-          float rr[4], ri[4], ir[4], ii[4];
-          const uint32_t c = c0 + 16 * i;
-          tmem_ld4_async(c, rr);            // A_re E_re
-          tmem_ld4_async(c + Np, ri);       // A_re E_im
-          tmem_ld4_async(c + 64, ir);       // A_im E_re
-          tmem_ld4_async(c + 64 + Np, ii);  // A_im E_im
-          tmem_ld_wait16(rr, ri, ir, ii);
-          pr[i] = make_float4(rr[0] - ii[0], rr[1] - ii[1], rr[2] - ii[2], rr[3] - ii[3]);
-          pi[i] = make_float4(ri[0] + ir[0], ri[1] + ir[1], ri[2] + ir[2], ri[3] + ir[3]);
-        }
+    // P of this row, group j
+    auto get_p = [&](uint32_t j, float4& re, float4& im) {
+      float rr[4], ri[4], ir[4], ii[4];
+      const uint32_t c = lanes + kColP + 4 * j, Np = 4 * n;
+      tmem_ld4_async(c, rr);            // A_re E_re
+      tmem_ld4_async(c + Np, ri);       // A_re E_im
+      tmem_ld4_async(c + 2 * kBlk, ir);       // A_im E_re
+      tmem_ld4_async(c + 2 * kBlk + Np, ii);  // A_im E_im
+      tmem_ld_wait16(rr, ri, ir, ii);
+      re = make_float4(rr[0] - ii[0], rr[1] - ii[1], rr[2] - ii[2], rr[3] - ii[3]);
+      im = make_float4(ri[0] + ir[0], ri[1] + ir[1], ri[2] + ir[2], ri[3] + ir[3]);
     };
     // four consecutive contraction columns of one row (re and im) into an
     // operand: rows f (re_hi), 32 + f, 64 + f, 96 + f
@@ -455,36 +467,30 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
       __syncwarp();
       if (lane == 0) mbar_arrive(bar);
     };
-    uint32_t gram_ph = 0, leg_ph = 0;  // parities of the MMAs waited for
+    uint32_t gram_ph = 0, leg_ph = 0, met_ph = 0;  // parities of the MMAs and meetings waited for
     auto gram_done = [&]() {
-      const bool r = wait(bar_done, gram_ph);
+      const bool r = wait(bar_done + 8u * target, gram_ph);
       gram_ph ^= 1u;
       return r;
     };
     auto leg_done = [&]() {
-      const bool r = wait(bar_leg_done, leg_ph);
+      const bool r = wait(bar_leg_done + 8u * target, leg_ph);
       leg_ph ^= 1u;
       return r;
     };
-    // One Gram stage: groups per s .. of every row.  A group's P is written by
-    // the warps that hold it, its V by those of (j + 2) % 4 == g (with two
-    // groups per stage the other ones), after the operands' last MMAs
-    // (`fresh`: there are none).
-    auto stage = [&](const float2* v, bool target_y, uint32_t n, uint32_t s, const float4& re, const float4& im, bool fresh) -> bool {
-      const uint32_t first = per * s, count = min(per, n - first);
-      const uint32_t jp = per == 4 ? g : g - first, jv = per == 4 ? (g + 2) & 3u : ((g + 2) & 3u) - first;  // within the stage
-      if (!fresh && !gram_done()) return false;
-      if (target_y ? in_y : in_x) {
-        unsigned char* op = g_op + (target_y ? op_y : op_x);
-        if (jv < count) {
-          float4 vr, vi;
-          if (!target_y || along_x) pr_row.template read<true>(v, target_y, first + jv, vr, vi);
-          else pr_row.template read<false>(v, target_y, first + jv, vr, vi);
-          put_op(op + kPairOp + jv * (P * pair_group(P)), vr, vi);
-        }
-        if (jp < count) put_op(op + jp * (P * pair_group(P)), re, im);
+    // One Gram stage, after the operands' last MMAs: this thread's groups
+    // 2 s + g of P and of V
+    auto stage = [&](const float2* v, uint32_t s) -> bool {
+      float4 re, im, vr, vi;
+      get_p(2 * s + g, re, im);
+      read4(v, 2 * s + g, vr, vi);
+      if (s > 0 && !gram_done()) return false;
+      if (in) {
+        unsigned char* op = ops + op_row + g * (P * pair_group(P));
+        put_op(op, re, im);
+        put_op(op + kOp, vr, vi);
       }
-      publish(bar_ready);
+      publish(bar_ready + 8u * target);
       return true;
     };
 
@@ -500,145 +506,130 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
       PairLayout<P> lay;
       lay.set(tk.L1 == 1, (uint32_t)tk.Dx, (uint32_t)tk.Dy);
       along_x = uniform(lay.along_x);
-      gx = lay.Xp / 4;
-      gy = lay.Yp / 4;
-      in_x = (uint32_t)row < P * lay.Xp;
-      in_y = (uint32_t)row < P * lay.Yp;
-      pr_row.set(lay, (uint32_t)row, g & 1u);
+      n = uniform(target ? lay.Xp : lay.Yp) / 4;
+      const uint32_t Np = target ? lay.Yp : lay.Xp;
+      in = (uint32_t)row < P * Np;
+      pr_row.set(lay, (uint32_t)row, g);
       uint32_t o, i;
-      lay.row((uint32_t)row, lay.Xp, o, i);
-      op_x = o * pair_group(P) + (i >> 3) * 128 + (i & 7) * 16;  // + P pair_group per group of four columns
-      lay.row((uint32_t)row, lay.Yp, o, i);
-      op_y = o * pair_group(P) + (i >> 3) * 128 + (i & 7) * 16;
-      build_pair_e<MR>(tk, e_op, lay.Xp, lay.Yp, warp, lane, kPairWarps);
+      lay.row((uint32_t)row, Np, o, i);
+      op_row = o * pair_group(P) + (i >> 3) * 128 + (i & 7) * 16;  // + P pair_group per group of four columns
+      build_pair_e<MR>(tk, e_op, lay.Xp, lay.Yp, (int)target, (int)target + 1, (int)w8, lane, kPairGroup);
     }
 #pragma unroll
-    for (int i = 0; i < 16; ++i) acc[0][i] = acc[1][i] = 0.0;
-    if ((ok = tile_ready(T))) {
-      put_a(raw + (size_t)(T & 1u) * 2 * kPairRawElems, false);
-      publish(bar_leg);
-    }
+    for (int i = 0; i < 32; ++i) acc[i] = 0.0;
     for (int t = 0; t < ntile && ok; ++t, ++T) {
-      const float2* wr = raw + (size_t)(T & 1u) * 2 * kPairRawElems;
-      const float2* vr = wr + kPairRawElems;
-      // what overlaps the MMAs of each stage is the work that follows it
-      if (!(ok = leg_done())) break;
-      get_p(gy);
-      if (!(ok = stage(vr, false, gy, 0, pr[0], pi[0], t == 0))) break;
-      put_a(wr, true);
-      publish(bar_leg);
-      if (gy > per && !(ok = stage(vr, false, gy, 1, pr[per / 4], pi[per / 4], false))) break;
-      if (t > 0) drain(acc[1], kColN + 128u);  // the last tile's Gram of y
-      if (!(ok = leg_done())) break;
-      get_p(gx);
-      if (!(ok = stage(vr, true, gx, 0, pr[0], pi[0], false))) break;
-      if (t + 1 < ntile) {
-        if (!(ok = tile_ready(T + 1))) break;
-        put_a(raw + (size_t)((T + 1) & 1u) * 2 * kPairRawElems, false);
-        publish(bar_leg);
+      const float2* wr = raw + (size_t)(T & 1u) * 2 * kRaw;
+      const float2* vr = wr + kRaw;
+      if (!kAhead || t == 0) {
+        if (!(ok = tile_ready(T))) break;
+        put_a(wr);
+        publish(bar_leg + 8u * target);
       }
-      drain(acc[0], kColN);
-      if (gx > per && !(ok = stage(vr, true, gx, 1, pr[per / 4], pi[per / 4], false))) break;
+      if (!(ok = leg_done())) break;
+      for (uint32_t s = 0; s < n / 2 && ok; ++s) ok = stage(vr, s);
+      if (!ok) break;
       if (lane == 0) mbar_arrive(bar_free + 8u * (T & 1u));
+      if (kAhead && t + 1 < ntile) {
+        if (!(ok = tile_ready(T + 1))) break;
+        put_a(raw + (size_t)((T + 1) & 1u) * 2 * kRaw);
+        publish(bar_leg + 8u * target);
+      }
+      if (!(ok = gram_done())) break;
+      drain();
     }
-    if (!ok || !(ok = gram_done())) break;
-    drain(acc[1], kColN + 128u);
-    // rows r and 64 + r of D, then N, through shared memory (the Gram
+    if (!ok) break;
+    // rows r and 64 + r of D, then N, through shared memory (the target's Gram
     // operands are free)
-    double* dsum = reinterpret_cast<double*>(g_op);  // 64 x 64
+    double* dsum = reinterpret_cast<double*>(ops);  // 64 x 64
+    auto meet = [&]() {  // the target's warps
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_group + 8u * target);
+      ok = wait(bar_group + 8u * target, met_ph);
+      met_ph ^= 1u;
+      return ok;
+    };
+    const int C = target == 0 ? tk.Dx : tk.Dy;
+    double2* part = (target == 0 ? tk.part_x : tk.part_y) + (long long)ch.chunk * C * C;
+    if (!meet()) break;
+    auto spill = [&](int half) {
+      if (row / 64 == half) {
 #pragma unroll
-    for (int target = 0; target < 2; ++target) {
-      const int C = target == 0 ? tk.Dx : tk.Dy;
-      double2* part = (target == 0 ? tk.part_x : tk.part_y) + (long long)ch.chunk * C * C;
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * kPairWarps) : "memory");
-      if (row >= 64) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) dsum[(row - 64) + 65 * (16 * (int)g + i)] = acc[target][i];
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * kPairWarps) : "memory");
-      if (row < 64) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) dsum[row + 65 * (16 * (int)g + i)] += acc[target][i];
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * kPairWarps) : "memory");
-      if (lane < C)
-        for (int c2 = warp; c2 < C; c2 += kPairWarps) {
-          const double re = dsum[lane + 65 * c2] + dsum[32 + lane + 65 * (32 + c2)];
-          const double im = dsum[32 + lane + 65 * c2] - dsum[lane + 65 * (32 + c2)];
-          part[lane + (long long)C * c2] = make_double2(re, im);
+        for (int i = 0; i < 32; ++i) {
+          double* d = dsum + (row & 63) + 65 * (8 * (i / 4) + 4 * (int)g + i % 4);
+          *d = half ? acc[i] : *d + acc[i];
         }
-    }
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * kPairWarps) : "memory");
+      }
+    };
+    spill(1);
+    if (!meet()) break;
+    spill(0);
+    if (!meet()) break;
+    if (lane < C)
+      for (int c2 = (int)w8; c2 < C; c2 += kPairGroup) {
+        const double re = dsum[lane + 65 * c2] + dsum[32 + lane + 65 * (32 + c2)];
+        const double im = dsum[32 + lane + 65 * c2] - dsum[lane + 65 * (32 + c2)];
+        part[lane + (long long)C * c2] = make_double2(re, im);
+      }
+    if (!meet()) break;
     }  // chunks
-    if (!ok && tid == 0) {
+    if (!ok && w8 == 0 && lane == 0) {
       // MMAs in flight get one more bounded wait before TMEM is freed
       atomicExch(&g_tc_error, 1);
-      mbar_wait(bar_leg_done, 0u);
-      mbar_wait(bar_leg_done, 1u);
-      mbar_wait(bar_done, 0u);
-      mbar_wait(bar_done, 1u);
+      for (uint32_t ph = 0; ph < 2; ++ph) {
+        mbar_wait(bar_leg_done + 8u * target, ph);
+        mbar_wait(bar_done + 8u * target, ph);
+      }
     }
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairRegsFeed));
-    if (warp == kPairWarps) {
-      // ---- the issuing warp: MMAs in the order in which the others publish
-      // One elected thread issues; every value that goes into an MMA is made
-      // warp-uniform first and the loops are unrolled, so that operands sit
-      // in uniform registers (left to per-thread registers each MMA took 170
-      // cycles to issue, three times its own time).
-      const uint32_t base = uniform(tmem), up = P, uper = per;
-      const uint32_t e0 = uniform(smem_u32(e_op)), g0 = uniform(smem_u32(g_op));
-      uint32_t gram_ph = 0, leg_ph = 0, nx = 0, ny = 0;
+    if (warp < kPairWarps + 2) {
+      // ---- the issuing warps, one per target: MMAs in the order in which
+      // its group publishes.  One elected thread issues; every value that
+      // goes into an MMA is made warp-uniform first and the loops are
+      // unrolled, so that operands sit in uniform registers (left to
+      // per-thread registers each MMA took 170 cycles to issue, three times
+      // its own time).
+      const uint32_t target = uniform((uint32_t)(warp - kPairWarps)), base = uniform(tmem) + 256u * target;
+      const uint32_t e0 = uniform(smem_u32(e_op)) + target * 2 * kPairE, g0 = uniform(smem_u32(g_op)) + target * 2 * kOp;
+      uint32_t gram_ph = 0, leg_ph = 0;
       bool ok = true;
-      auto leg = [&](uint32_t which) {  // 0: E_y (K = Yp), 1: E_x
-        ok = wait(bar_leg, leg_ph);
-        leg_ph ^= 1u;
-        if (!ok) return;
-        const uint32_t k8 = (which ? nx : ny) / 2, N2 = 16 * k8, idesc = idesc_tf32(128, 0) | ((N2 >> 3) << 17);
-        const uint64_t dh0 = smem_desc(e0 + which * 2 * kPairE, N2 * 16, 128), dl0 = smem_desc(e0 + which * 2 * kPairE + kPairE, N2 * 16, 128);
-        if (elect_one()) {
-#pragma unroll
-          for (uint32_t part = 0; part < 2; ++part)
-#pragma unroll
-            for (uint32_t s = 0; s < 4; ++s)
-              if (s < k8) {
-                const uint32_t d = base + kColP + 64u * part, ah = base + 32u * part + 8u * s;
-                const uint64_t dh = dh0 + s * 2 * N2, dl = dl0 + s * 2 * N2;  // two 16-byte K groups of N2 rows
-                mma_tf32_ts(d, ah, dh, idesc, s);
-                mma_tf32_ts(d, ah, dl, idesc, 1u);
-                mma_tf32_ts(d, ah + 64u, dh, idesc, 1u);
-              }
-          mma_commit(bar_leg_done);
-        }
-        __syncwarp();
-      };
-      const uint64_t da = smem_desc(g0, pair_group(P), 128), db = smem_desc(g0 + kPairOp, pair_group(P), 128);
-      auto stage = [&](uint32_t target, uint32_t count, uint32_t accumulate) {
-        ok = wait(bar_ready, gram_ph);
-        gram_ph ^= 1u;
-        if (!ok) return;
-        const uint32_t idesc = idesc_tf32(128, 128), d = base + kColN + 128u * target, ks = up * count / 2;
-        if (elect_one()) {
-#pragma unroll
-          for (uint32_t s = 0; s < 8; ++s)
-            if (s < ks) mma_tf32(d, da + pair_group(P) / 8 * s, db + pair_group(P) / 8 * s, idesc, accumulate + s);
-          mma_commit(bar_done);
-        }
-        __syncwarp();
-      };
+      const uint64_t da = smem_desc(g0, pair_group(P), 128), db = smem_desc(g0 + kOp, pair_group(P), 128);
       for (PairChunks ch(tasks, begins, ntask, first_tile, last_tile); ok && ch.valid(); ++ch.chunk) {
         const LegPairTask& tk = tasks[ch.ti];
         const int ntile = min(tk.chunk_tiles, (int)((tk.n_outer + P - 1) / P) - ch.chunk * tk.chunk_tiles);
-        nx = uniform(2u * (((uint32_t)tk.Dx + 7u) >> 3));
-        ny = uniform(2u * (((uint32_t)tk.Dy + 7u) >> 3));
-        leg(0);
+        // target x absorbs E_y (K = Yp), y E_x
+        const uint32_t k8 = uniform(((uint32_t)(target ? tk.Dx : tk.Dy) + 7u) >> 3), N2 = 16 * k8;
         for (int t = 0; t < ntile && ok; ++t) {
-          stage(0, min(uper, ny), 0u);
-          if (ok) leg(1);
-          if (ok && ny > uper) stage(0, ny - uper, 1u);
-          if (ok) stage(1, min(uper, nx), 0u);
-          if (ok && t + 1 < ntile) leg(0);
-          if (ok && nx > uper) stage(1, nx - uper, 1u);
+          if (!(ok = wait(bar_leg + 8u * target, leg_ph))) break;
+          leg_ph ^= 1u;
+          const uint32_t idesc = idesc_tf32(128, 0) | ((N2 >> 3) << 17);
+          const uint64_t dh0 = smem_desc(e0, N2 * 16, 128), dl0 = smem_desc(e0 + kPairE, N2 * 16, 128);
+          if (elect_one()) {
+#pragma unroll
+            for (uint32_t part = 0; part < 2; ++part)
+#pragma unroll
+              for (uint32_t s = 0; s < kBlk / 8; ++s)
+                if (s < k8) {
+                  const uint32_t d = base + kColP + 2 * kBlk * part, ah = base + kBlk * part + 8u * s;
+                  const uint64_t dh = dh0 + s * 2 * N2, dl = dl0 + s * 2 * N2;  // two 16-byte K groups of N2 rows
+                  mma_tf32_ts(d, ah, dh, idesc, s);
+                  mma_tf32_ts(d, ah, dl, idesc, 1u);
+                  mma_tf32_ts(d, ah + 2 * kBlk, dh, idesc, 1u);
+                }
+            mma_commit(bar_leg_done + 8u * target);
+          }
+          __syncwarp();
+          for (uint32_t st = 0; st < k8; ++st) {
+            if (!(ok = wait(bar_ready + 8u * target, gram_ph))) break;
+            gram_ph ^= 1u;
+            if (elect_one()) {
+#pragma unroll
+              for (uint32_t s = 0; s < P; ++s)
+                mma_tf32(base + kColN, da + pair_group(P) / 8 * s, db + pair_group(P) / 8 * s, idesc_tf32(128, 128), st + s);
+              mma_commit(bar_done + 8u * target);
+            }
+            __syncwarp();
+          }
         }
       }
     } else {
@@ -646,7 +637,7 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
       // memory, one or two elements per copy; padding is written as zeros
       uint32_t T = 0;
       bool ok = true;
-      const uint32_t y0 = (uint32_t)(warp - kPairWarps - 1);
+      const uint32_t y0 = (uint32_t)(warp - kPairWarps - 2);
       for (PairChunks ch(tasks, begins, ntask, first_tile, last_tile); ok && ch.valid(); ++ch.chunk) {
         const LegPairTask& tk = tasks[ch.ti];
         const int ntile = min(tk.chunk_tiles, (int)((tk.n_outer + P - 1) / P) - ch.chunk * tk.chunk_tiles);
@@ -672,10 +663,10 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
               float2* de = d + (e ^ lay.swz(y));
               if constexpr (w == 2) {
                 cp16(de, in ? p : Wg, in);
-                cp16(de + kPairRawElems, in ? p + VmW : Wg, in);
+                cp16(de + kRaw, in ? p + VmW : Wg, in);
               } else {
                 cp8(de, in ? p : Wg, in);
-                cp8(de + kPairRawElems, in ? p + VmW : Wg, in);
+                cp8(de + kRaw, in ? p + VmW : Wg, in);
               }
               p += dy;
               d += kPairLoaders * lay.PE;
@@ -686,7 +677,7 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
         for (int t = 0; t < ntile && ok; ++t, ++T) {
           const uint32_t st = T & 1u;
           if (T >= 2 && !(ok = wait(bar_free + 8u * st, ((T >> 1) - 1) & 1u))) break;
-          float2* dst = raw + (size_t)st * 2 * kPairRawElems;
+          float2* dst = raw + (size_t)st * 2 * kRaw;
           const uint32_t o0 = (uint32_t)(ch.chunk * tk.chunk_tiles + t) * P;
           if (wide) copy(std::integral_constant<uint32_t, 2>{}, dst, o0);
           else copy(std::integral_constant<uint32_t, 1>{}, dst, o0);
@@ -938,7 +929,7 @@ __device__ __forceinline__ void pair_absorb(const LegPairTask* __restrict__ task
       src = static_cast<const float2*>(tk.V);
       dst = static_cast<const float2*>(tk.W) - src;
       loaded = false;
-      build_pair_e<MR>(tk, e_op, lay.Xp, lay.Yp, warp, lane, kAbsorbThreads / 32);
+      build_pair_e<MR>(tk, e_op, lay.Xp, lay.Yp, 0, 2, warp, lane, kAbsorbThreads / 32);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (!loaded) {

@@ -40,3 +40,13 @@ def test_wide_site_matches_oracle(dims, prec):
         st.set_state(V, E)
         tb.BeliefPropagation(st)
         assert max(float(np.max(np.abs(st.get_message(m) - F[m]))) for m in range(2 * ne)) <= 3.5e-5
+
+
+# Even extents that end inside a group of four columns, tiles that are not full
+FORMS = [(50, 3), (34, 7, 3), (42, 38, 35), (6, 9, 34, 2)]
+
+
+@pytest.mark.parametrize("prec", [tb.MIXED, tb.C64], ids=["mixed", "c64"])
+@pytest.mark.parametrize("dims", FORMS, ids=["x".join(map(str, d)) for d in FORMS])
+def test_memory_forms_match_oracle(dims, prec):
+    test_wide_site_matches_oracle(dims, prec)

@@ -11,8 +11,8 @@
 // M: [M_re | M_im], D1 = A_re M', D2 = A_im M'), K in two halves with an
 // operand each, so that the next tile's first half is converted during this
 // tile's second MMAs; the result returns over the tile it came from and is
-// written out as memory runs.  Per 5x5 sweep at D = 64: 24.9 -> 10.8 ms (9000
-// cycles per tile, 4 TB/s; 11000 at L = 1, whose tiles go out through shared
+// written out as memory runs.  Per 5x5 sweep at D = 64: 24.9 -> 10.2 ms (9000
+// cycles per tile, 4 TB/s; 9400 at L = 1, whose tiles go out through shared
 // memory).
 //
 // 512 threads, persistent, one CTA per SM (194 KB of shared memory, all of
@@ -29,7 +29,7 @@ namespace tc {
 
 constexpr int kTcMaxD64 = 64;
 constexpr int kLeg64Threads = 512;
-constexpr int kLeg64Pitch = kTcRows + 1;  // element (row, j) of a tile at j pitch + row: odd
+constexpr int kLeg64Pitch = kTcRows + 1;  // of a tile's columns: odd, see leg64_form
 constexpr uint32_t kLeg64Op = 128 * 64 * 4;
 
 __host__ __device__ constexpr size_t leg64_smem_bytes() {
@@ -44,6 +44,19 @@ __host__ __device__ inline int leg64_rows(long long L) { return L <= 32 ? (int)(
 __host__ __device__ inline long long leg64_tiles(long long L, long long R) {
   const long long rows = leg64_rows(L);
   return (L * R + rows - 1) / rows;
+}
+
+// How a tile lies in shared memory.  Rows that are contiguous in memory (L =
+// 1, even dimensions) stay rows of 64, pairs swizzled by the row; where lanes
+// run along memory (even L above 32) element (row, j) lies at 128 j + row.
+// Both are copied 16 bytes at a time, and read without bank conflicts (D =
+// 64, cycles per tile: 10900 -> 9400 at L = 1, 9300 -> 9100 above).  The
+// rest, at 129 j + row, takes eight.
+enum : uint32_t { kLeg64Any, kLeg64Row, kLeg64Col };
+__device__ __forceinline__ uint32_t leg64_form(const LegTask& t) {
+  if ((reinterpret_cast<uintptr_t>(t.in) | reinterpret_cast<uintptr_t>(t.out)) & 15) return kLeg64Any;
+  if (t.L == 1) return ((t.Din | t.Dout) & 1) == 0 ? kLeg64Row : kLeg64Any;
+  return t.L > 32 && (t.L & 1) == 0 ? kLeg64Col : kLeg64Any;
 }
 
 }  // namespace tc
@@ -90,12 +103,33 @@ __global__ void __launch_bounds__(tc::kLeg64Threads, 1) k_leg_apply_tc64(const L
   // of the current task
   LegTask tk{};
   uint32_t L = 1, rows = 0, rpt = kTcRows, Din = 0, Dout = 0, Np = 8, nk = 1, nk0 = 1;  // K steps of 8, of the first half
+  uint32_t form = kLeg64Any, pitch = kLeg64Pitch;
+  const uint32_t swz = 2 * ((uint32_t)row & 7), at_row = 64 * (uint32_t)row;  // kLeg64Row
 
   auto load_tile = [&](uint32_t lt, int stage) {
     float2* d = raw + (size_t)stage * kTcMaxD64 * kLeg64Pitch;
     const float2* in = static_cast<const float2*>(tk.in);
     const uint32_t q0 = lt * rpt, n = min(rpt, rows - q0);
-    if (L <= 32) {
+    if (form == kLeg64Row) {
+      const float2* p = in + (size_t)q0 * Din;
+      for (uint32_t i = 2 * (uint32_t)tid; i < n * Din; i += 2 * kLeg64Threads) {
+        const uint32_t r = fast_div(i, tk.div_din), j = i - r * Din;
+        cp16(d + 64 * r + (j ^ (2 * (r & 7))), p + i, true);
+      }
+    } else if (form == kLeg64Col) {
+      const uint32_t i = 2 * ((uint32_t)tid & 63), j0 = (uint32_t)tid >> 6;
+      if (i < n) {
+        const uint32_t q = q0 + i, r = fast_div(q, tk.div_l), l = q - r * L;
+        const float2* p = in + (size_t)l + (size_t)L * ((size_t)Din * r + j0);
+        float2* e = d + j0 * kTcRows + i;
+#pragma unroll 4
+        for (uint32_t j = j0; j < Din; j += 8) {
+          cp16(e, p, true);
+          p += (size_t)L * 8;
+          e += 8 * kTcRows;
+        }
+      }
+    } else if (L <= 32) {
       const float2* p = in + (size_t)q0 * Din;
       for (uint32_t i = (uint32_t)tid; i < n * Din; i += kLeg64Threads) {
         const uint32_t c = fast_div(i, tk.div_l), l = i - c * L, r = fast_div(c, tk.div_din), j = c - r * Din;
@@ -115,6 +149,23 @@ __global__ void __launch_bounds__(tc::kLeg64Threads, 1) k_leg_apply_tc64(const L
     // this thread's arrival, when its copies have landed
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar_full + 8u * stage) : "memory");
   };
+  // columns j .. j + 3 of this row, zero from Din on
+  auto read4 = [&](const float2* t, uint32_t j, float2* e) {
+    if (form == kLeg64Row) {
+      const uint32_t i = at_row + (j ^ swz);
+      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 a = j < Din ? *reinterpret_cast<const float4*>(t + i) : z;
+      const float4 b = j + 2 < Din ? *reinterpret_cast<const float4*>(t + (i ^ 2)) : z;
+      e[0] = make_float2(a.x, a.y);
+      e[1] = make_float2(a.z, a.w);
+      e[2] = make_float2(b.x, b.y);
+      e[3] = make_float2(b.z, b.w);
+      return;
+    }
+    const float2* p = t + j * pitch + row;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) e[k] = j + k < Din ? p[k * pitch] : make_float2(0.f, 0.f);
+  };
   auto put_a = [&](const float2* t, uint32_t half) {
     const uint32_t j0 = half ? 2 * nk0 : 0, n = 2 * (half ? nk - nk0 : nk0);  // groups
     const uint32_t a = lanes + 128 * half;
@@ -122,10 +173,8 @@ __global__ void __launch_bounds__(tc::kLeg64Threads, 1) k_leg_apply_tc64(const L
     for (uint32_t i = g; i < 8; i += 4)
       if (i < n) {
         const uint32_t j = 4 * (j0 + i);
-        const float2* p = t + j * kLeg64Pitch + row;
         float2 e[4];
-#pragma unroll
-        for (uint32_t k = 0; k < 4; ++k) e[k] = j + k < Din ? p[k * kLeg64Pitch] : make_float2(0.f, 0.f);
+        read4(t, j, e);
         float4 rh, rl, ih, il;
         split4(make_float4(e[0].x, e[1].x, e[2].x, e[3].x), rh, rl);
         split4(make_float4(e[0].y, e[1].y, e[2].y, e[3].y), ih, il);
@@ -213,6 +262,8 @@ __global__ void __launch_bounds__(tc::kLeg64Threads, 1) k_leg_apply_tc64(const L
       Np = (Dout + 7u) & ~7u;
       nk = (Din + 7u) / 8;
       nk0 = (nk + 1) / 2;
+      form = uniform(leg64_form(tk));
+      pitch = form == kLeg64Col ? kTcRows : kLeg64Pitch;
       task_end = begins[ti] + leg64_tiles(tk.L, tk.R);
       lt = (uint32_t)(tile - begins[ti]);
       loaded = halved = false;
@@ -276,7 +327,11 @@ __global__ void __launch_bounds__(tc::kLeg64Threads, 1) k_leg_apply_tc64(const L
         tmem_ld4_async(c + 128, ir);       // A_im M_re
         tmem_ld4_async(c + 128 + Np, ii);  // A_im M_im
         tmem_ld_wait16(rr, ri, ir, ii);
-        if ((uint32_t)row < n) {
+        if ((uint32_t)row < n && form == kLeg64Row) {
+          float2* p = t + at_row;
+          *reinterpret_cast<float4*>(p + ((4 * i) ^ swz)) = make_float4(rr[0] - ii[0], ri[0] + ir[0], rr[1] - ii[1], ri[1] + ir[1]);
+          *reinterpret_cast<float4*>(p + ((4 * i + 2) ^ swz)) = make_float4(rr[2] - ii[2], ri[2] + ir[2], rr[3] - ii[3], ri[3] + ir[3]);
+        } else if ((uint32_t)row < n) {
 #pragma unroll
           for (uint32_t k = 0; k < 4; ++k) {
             const float2 v = make_float2(rr[k] - ii[k], ri[k] + ir[k]);
@@ -288,6 +343,12 @@ __global__ void __launch_bounds__(tc::kLeg64Threads, 1) k_leg_apply_tc64(const L
     if (!direct) {
       __syncthreads();
       float2* o = out + (size_t)q0 * Dout;
+      if (form == kLeg64Row) {
+        for (uint32_t i = 2 * (uint32_t)tid; i < n * Dout; i += 2 * kLeg64Threads) {
+          const uint32_t r = Dout == Din ? fast_div(i, tk.div_din) : i / Dout, k = i - r * Dout;
+          *reinterpret_cast<float4*>(o + i) = *reinterpret_cast<const float4*>(t + 64 * r + (k ^ (2 * (r & 7))));
+        }
+      } else
       for (uint32_t i = (uint32_t)tid; i < n * Dout; i += kLeg64Threads) {
         const uint32_t c = fast_div(i, tk.div_l), l = i - c * L;
         const uint32_t r = Dout == Din ? fast_div(c, tk.div_din) : c / Dout, k = c - r * Dout;

@@ -15,7 +15,10 @@
 // alternate between two operand buffers and 64-row sums between two
 // accumulators, so loads (two tiles ahead, in registers), conversion, MMAs
 // and the FP64 additions of finished sums overlap, and warps meet only through
-// barriers of the operands.  Per 5x5 sweep at D = 64: 14.3 -> 6.5 ms (3 TB/s).
+// barriers of the operands.  A thread's four rows of a column come in one
+// 32-byte load (in two of 16 each half of every sector: 3250 -> 2700 cycles
+// per 32 rows at L > 1; 2600 at L = 1).  Per 5x5 sweep at D = 64: 14.3 -> 5.8
+// ms (3.4 TB/s).
 //
 // One CTA (512 threads) per split-K chunk.  Every wait is bounded: on timeout
 // the CTA records g_tc_error, waits once more (bounded) for its MMAs, frees
@@ -32,6 +35,12 @@ constexpr int kGram64Q = 32;                    // contraction rows per tile
 constexpr uint32_t kGram64X = 128 * kGram64Q * 4;  // X_hi or X_lo of a tile; Y (256 rows) is twice that
 __host__ __device__ constexpr size_t gram64_smem_bytes() { return 1024 + 8 * (size_t)kGram64X + 64; }
 __host__ __device__ inline bool gram64_ok(int C, int P) { return P == 1 && C > kTcMaxD && C <= 64; }
+// 32 aligned bytes, a whole sector, in one load
+__device__ __forceinline__ void ldg32(const float2* p, float4& a, float4& b) {
+  asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+               : "l"(p));
+}
 }  // namespace tc
 
 __global__ void __launch_bounds__(tc::kGram64Threads, 1) k_gram_tc64(const GramTask* __restrict__ tasks,
@@ -73,6 +82,8 @@ __global__ void __launch_bounds__(tc::kGram64Threads, 1) k_gram_tc64(const GramT
   const uint32_t place = q4 * (128 * 16) + (c >> 3) * 128 + (c & 7) * 16;   // X: 128 rows
   const uint32_t place_y = q4 * (256 * 16) + (c >> 3) * 128 + (c & 7) * 16;  // Y: 256 rows
   const bool mine = c < (uint32_t)C;
+  // four rows of a column are 32 contiguous, aligned bytes
+  const bool wide = (L & 3) == 0 && ((reinterpret_cast<uintptr_t>(tk.A) | reinterpret_cast<uintptr_t>(tk.B)) & 31) == 0;
   const float2* __restrict__ A = static_cast<const float2*>(tk.A) + (size_t)L * c;
   const float2* __restrict__ B = static_cast<const float2*>(tk.B) + (size_t)L * c;
 
@@ -99,14 +110,10 @@ __global__ void __launch_bounds__(tc::kGram64Threads, 1) k_gram_tc64(const GramT
     }
     p.a01 = p.a23 = p.b01 = p.b23 = make_float4(0.f, 0.f, 0.f, 0.f);
     if (!mine) return;
-    if ((L & 3) == 0 && q + 3 < qend) {  // 32 contiguous, aligned bytes
+    if (wide && q + 3 < qend) {
       const size_t off = (size_t)l + (size_t)LC * m;
-      const float4* pa = reinterpret_cast<const float4*>(A + off);
-      const float4* pb = reinterpret_cast<const float4*>(B + off);
-      p.a01 = __ldg(pa);
-      p.a23 = __ldg(pa + 1);
-      p.b01 = __ldg(pb);
-      p.b23 = __ldg(pb + 1);
+      ldg32(A + off, p.a01, p.a23);
+      ldg32(B + off, p.b01, p.b23);
       return;
     }
     float2 a[4], b[4];

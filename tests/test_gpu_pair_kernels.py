@@ -40,7 +40,7 @@ def test_degree_four_site_matches_oracle(dims, prec):
         for _ in range(2):  # twice from the same messages: nothing is left behind
             for m in range(8):
                 st.set_message(m, E[m])
-            tb.BeliefPropagation(st)
+            tb.BeliefPropagationLoop(st, 1e-300, 1)  # its sweeps take pairs of legs
             got = [st.get_message(m) for m in range(8)]
             assert max(float(np.max(np.abs(a - b))) for a, b in zip(got, F)) <= 2e-5
 

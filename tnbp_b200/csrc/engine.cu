@@ -723,7 +723,18 @@ void Job::autotune_waves() {
   if (f) f << key << '\t' << best_mb << '\t' << best_ms << '\t' << default_ms << '\n';
 }
 
-void Job::build_plan() {
+// The loop's sweeps take degree-4 sites by pairs of legs, single sweeps leg by
+// leg: the two agree to the rounding of 32-bit products (6e-7), and a loop
+// ends where that no longer matters, but sweeps that a program counts itself
+// may run on messages far from any fixed point, where loopy BP amplifies
+// rounding (random states: 600 to 1000 times in four sweeps).  Their results
+// do not depend on how fast a loop is.  36 sites at D = 32, d = 2, per sweep:
+// 5.8 ms leg by leg, 2.4 ms in pairs.
+void Job::ensure_plan(bool pairs) {
+  if (!plan.valid || (plan.pairable && plan.pairs != pairs)) build_plan(pairs);
+}
+
+void Job::build_plan(bool pairs) {
   TNBP_TRACE_SCOPE("sweep.build_plan");
   {
     TNBP_TRACE_SCOPE("sweep.build_plan.release");
@@ -759,7 +770,10 @@ void Job::build_plan() {
       return reduced_sweeps(prec) && tcgen05_enabled() && leg_gram_enabled() && tc::leg_gram_ok(sh[t], sh[w]);
     };
     const int nunits = gs >= 2 ? 2 : 1;
-    const bool pair = reduced_sweeps(prec) && tcgen05_enabled() && !leg_gram_enabled() && tc::pair_ok(sh.data(), gs);
+    const bool can_pair =
+        reduced_sweeps(prec) && tcgen05_enabled() && !leg_gram_enabled() && !bulk_leg_enabled() && tc::pair_ok(sh.data(), gs);
+    const bool pair = pairs && can_pair;
+    plan.pairable = plan.pairable || can_pair;
     for (int u = 0; u < nunits; ++u)
       units.push_back(pair ? make_pair_unit(s, u) : make_unit(s, u, ops, sp, fuse));
   }
@@ -1022,6 +1036,7 @@ void Job::build_plan() {
       plan.msg[par].push_back(m);
     }
   }
+  plan.pairs = pairs;
   plan.valid = true;
   static std::atomic<uint64_t> serials{0};
   plan_serial = ++serials;
@@ -1082,12 +1097,14 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
     tiles[k] += (t.n_outer + t.planes - 1) / t.planes;
     pt[k].push_back(t);
   };
-  // The kernel is chosen per task, never per launch: complex64 tasks whose
-  // tile is a contiguous byte range (tc::bulk_mode) run on the bulk-staged
-  // tcgen05 kernel, other tasks with Din, Dout <= 32 on the register-staged
-  // tcgen05 kernel, every other task on the CUDA-core kernel, whatever else
-  // shares the batch.  A request's rounding therefore does not depend on
-  // what it is batched with.
+  // The kernel is chosen per task, never per launch.  Complex64 sites of
+  // degree 4 with dimensions up to 32 come as pairs of legs; other complex64
+  // leg tasks run, if opted in and a tile is a contiguous byte range
+  // (tc::bulk_mode), on the bulk-staged tcgen05 kernel, with a dimension of 33
+  // to 64 on the 64-wide one, with smaller ones on the register-staged one,
+  // above on the CUDA cores; complex128 tasks on the FP64 tensor kernel,
+  // whatever else shares the batch.  A request's rounding therefore does not
+  // depend on what it is batched with.
   const bool reduced = !entries.empty() && reduced_sweeps(entries[0].job->prec);
   const bool tc_ok = reduced && tcgen05_enabled();
   {
@@ -1442,8 +1459,8 @@ bool leg_gram_enabled() {
 }
 
 // Every site whose tensor, two work buffers, messages and Gram partials fit
-// kSiteSmemMax of shared memory is swept on chip, one CTA per message (k_site_sweep);
-// the other sites take the per-level path.  Measured on the random-circuit
+// kSiteSmemMax of shared memory is swept on chip, one CTA per message
+// (k_site_sweep); the other sites take the per-level path.  Measured on the random-circuit
 // workload (10x10, BP at D <= 8): BP loops 4.6-5.7 ms per solve against
 // 23-33 ms per-level (mixed), 4.9-6.3 against 8.0-8.5 ms (complex128); the
 // 16x16 headline unchanged within run-to-run noise.  TNBP_SITE_SWEEP=0
@@ -1540,6 +1557,8 @@ double Job::read_cond() {
   return host_scalar[0];
 }
 void Job::bp_sweep() {
+  sync_shadow();
+  ensure_plan(false);
   run_sweep(cur);
   cur = 1 - cur;
   CK(cudaStreamSynchronize(stream));
@@ -1547,6 +1566,8 @@ void Job::bp_sweep() {
 }
 
 double Job::bp_condition() {
+  sync_shadow();
+  ensure_plan(false);
   run_sweep(cur);  // writes the other arena; state (cur) unchanged
   return read_cond();
 }
@@ -1579,7 +1600,7 @@ void Job::bp_run(double tol_in, int max_iter, int* iters, double* cond) {
   *cond = std::nan("");
   if (max_iter <= 0) return;
   sync_shadow();
-  if (!plan.valid) build_plan();
+  ensure_plan(true);
   autotune_waves();
   run_sweep(cur);
   cur = 1 - cur;

@@ -118,6 +118,8 @@ struct SweepBatch {
 
 struct SweepPlan {
   bool valid = false;
+  bool pairs = false;     // degree-4 sites by pairs of legs, where they can be
+  bool pairable = false;  // some can
   DevBuf partial, dist;
   std::vector<WaveHost> waves;
   std::vector<GramTask> gram;
@@ -254,7 +256,9 @@ struct Job {
   void sync_shadow();
   void* mptr(int arena, int m) const;
   void destroy_graphs();
-  void build_plan();
+  void build_plan(bool pairs = true);
+  // A plan for the loop's sweeps (pairs) or for single sweeps.
+  void ensure_plan(bool pairs);
   size_t scratch_limit() const;
   void run_sweep(int par);
   double read_cond();

@@ -291,7 +291,7 @@ Server::GroupSweep Server::prepare_group(int gprec, const std::vector<Request*>&
   std::vector<BatchEntry> entries;
   for (auto* r : inbp) {
     r->job->sync_shadow();
-    if (!r->job->plan.valid) r->job->build_plan();
+    r->job->ensure_plan(true);
     entries.push_back({r->job.get(), r->job->cur});
   }
   prepare_kernels(gprec);

@@ -628,7 +628,7 @@ def run_ours(args, rank, world, local_rank):
         "clocks": clk.summary(),
     }
     line["roofline"] = {
-        "kernel": "BP sweep (k_leg_apply_tc + k_gram_tc + k_msg_finalize + k_segmented_sum, one CUDA graph)",
+        "kernel": "BP sweep (k_pair_absorb_tc + k_pair_gram_tc + k_leg_apply_tc + k_gram_tc + k_msg_finalize + k_segmented_sum, one CUDA graph)",
         "bound": "tensor",
         "achieved": achieved,
         "peak": tf_peak,
@@ -642,9 +642,9 @@ def run_ours(args, rank, world, local_rank):
                         "hbm_achieved_gbs": (tot_by / n_sw) / ((tot_ms / n_sw) / 1e3) / 1e9 if n_sw else None,
                         "hbm_peak_gbs": peaks.get("hbm_gbs")},
     }
-    # the DRAM bytes the unfused schedule moves per D = 32 sweep (ncu, scaled
-    # from the 5x5 capture) over the measured sweep time: how close the
-    # kernels run to the copy bandwidth on the traffic they must move
+    # the DRAM bytes that the sweep's schedule moves at D = 32 (computed, see
+    # the file) over the measured sweep time: how close the kernels run to the
+    # copy bandwidth on the traffic they must move
     if traffic and n_sw and peaks.get("hbm_gbs"):
         rate = traffic / ((tot_ms / n_sw) / 1e3) / 1e9
         line["roofline"]["schedule_traffic"] = {"gbs": rate, "frac_of_hbm": rate / peaks["hbm_gbs"],

@@ -54,3 +54,26 @@ FORMS = [(1, 1, 32, 32), (1, 1, 17, 9), (2, 1, 9, 8), (3, 1, 32, 32), (2, 5, 16,
 @pytest.mark.parametrize("dims", FORMS, ids=["x".join(map(str, d)) for d in FORMS])
 def test_memory_forms_match_oracle(dims, prec):
     test_degree_four_site_matches_oracle(dims, prec)
+
+
+@pytest.mark.parametrize("prec", [tb.MIXED, tb.C64], ids=["mixed", "c64"])
+def test_single_sweeps_do_not_depend_on_the_loop(prec):
+    """A sweep between loops gives the bits of a sweep without one."""
+    if not tb.device_available():
+        pytest.fail("no CUDA device: the GPU tests need a B200")
+    rng = np.random.default_rng(7)
+    dims = (16, 12, 9, 20)
+    edges = [(0, k + 1) for k in range(4)]
+    gauss = lambda sh: rng.normal(size=sh) + 1j * rng.normal(size=sh)
+    V = [gauss([dims[m] for m in bn.bonds_of(edges, s)] + [2]) for s in bn.sites_of(edges)]
+    E = [np.eye(dims[m % 4]) / np.sqrt(dims[m % 4]) for m in range(8)]
+    with tb.State(edges, prec) as st:
+        st.set_state(V, E)
+        out = []
+        for step in (tb.BeliefPropagation, lambda s: tb.BeliefPropagationLoop(s, 1e-300, 1), tb.BeliefPropagation):
+            for m in range(8):
+                st.set_message(m, E[m])
+            step(st)
+            out.append([st.get_message(m) for m in range(8)])
+        assert all(np.array_equal(a, b) for a, b in zip(out[0], out[2]))
+        assert max(float(np.max(np.abs(a - b))) for a, b in zip(out[0], out[1])) <= 2e-5

@@ -442,6 +442,7 @@ struct Unit {
   std::vector<Fused> fused;  // targets with the fused absorption + Gram
   int pair_src = -2;         // slot of W for the unit's pair of targets (k_pair_gram_tc); -2: none
   int pair = 0;              // the targets are legs 2 pair and 2 pair + 1
+  bool f64 = false;          // in complex128, from V itself
   std::map<int, int> buf_of_slot;
   int nbuf = 0;
   int nlevels = 0;
@@ -723,18 +724,19 @@ void Job::autotune_waves() {
   if (f) f << key << '\t' << best_mb << '\t' << best_ms << '\t' << default_ms << '\n';
 }
 
-// The loop's sweeps take degree-4 sites by pairs of legs, single sweeps leg by
-// leg: the two agree to the rounding of 32-bit products (6e-7), and a loop
-// ends where that no longer matters, but sweeps that a program counts itself
-// may run on messages far from any fixed point, where loopy BP amplifies
-// rounding (random states: 600 to 1000 times in four sweeps).  Their results
-// do not depend on how fast a loop is.  36 sites at D = 32, d = 2, per sweep:
-// 5.8 ms leg by leg, 2.4 ms in pairs.
-void Job::ensure_plan(bool pairs) {
-  if (!plan.valid || (plan.pairable && plan.pairs != pairs)) build_plan(pairs);
+// The loop's sweeps take degree-4 sites by pairs of legs and the mixed path's
+// small sites in complex128, single sweeps leg by leg: the two agree to the
+// rounding of 32-bit products (6e-7), and a loop ends where that no longer
+// matters, but sweeps that a program counts itself may run on messages far
+// from any fixed point, where loopy BP amplifies rounding (random states: 600
+// to 1000 times in four sweeps).  Their results do not depend on how fast a
+// loop is.  36 sites at D = 32, d = 2, per sweep: 5.8 ms leg by leg, 2.4 ms in
+// pairs.
+void Job::ensure_plan(bool loop) {
+  if (!plan.valid || (plan.varies && plan.loop != loop)) build_plan(loop);
 }
 
-void Job::build_plan(bool pairs) {
+void Job::build_plan(bool loop) {
   TNBP_TRACE_SCOPE("sweep.build_plan");
   {
     TNBP_TRACE_SCOPE("sweep.build_plan.release");
@@ -751,6 +753,7 @@ void Job::build_plan(bool pairs) {
     const int gs = (int)g.legs[s].size();
     if (site_whole(s)) {
       small_sites.push_back(s);
+      plan.varies = plan.varies || prec == TNBP_MIXED;
       continue;
     }
     std::vector<PlanOp> ops;
@@ -764,18 +767,21 @@ void Job::build_plan(bool pairs) {
     sp.rec(-1, 0, -1, targets, std::vector<char>(gs, 0), gs);
     result[s] = sp.result;
     const auto sh = site_shape(s);
+    const bool f64 = prec == TNBP_C128 || (loop && site_f64(s));
     // the last absorption of a target runs fused with its Gram on tcgen05
     // (complex64 sweeps, both dims <= 32); decided from this job alone
     auto fuse = [&](int t, int w) {
-      return reduced_sweeps(prec) && tcgen05_enabled() && leg_gram_enabled() && tc::leg_gram_ok(sh[t], sh[w]);
+      return !f64 && reduced_sweeps(prec) && tcgen05_enabled() && leg_gram_enabled() && tc::leg_gram_ok(sh[t], sh[w]);
     };
     const int nunits = gs >= 2 ? 2 : 1;
     const bool can_pair =
-        reduced_sweeps(prec) && tcgen05_enabled() && !leg_gram_enabled() && !bulk_leg_enabled() && tc::pair_ok(sh.data(), gs);
-    const bool pair = pairs && can_pair;
-    plan.pairable = plan.pairable || can_pair;
-    for (int u = 0; u < nunits; ++u)
+        !site_f64(s) && reduced_sweeps(prec) && tcgen05_enabled() && !leg_gram_enabled() && !bulk_leg_enabled() && tc::pair_ok(sh.data(), gs);
+    const bool pair = loop && can_pair;
+    plan.varies = plan.varies || can_pair || site_f64(s);
+    for (int u = 0; u < nunits; ++u) {
       units.push_back(pair ? make_pair_unit(s, u) : make_unit(s, u, ops, sp, fuse));
+      units.back().f64 = f64;
+    }
   }
   // 2. waves of consecutive units within the byte budget (at least one unit)
   if (!tuning) choose_wave_budget();
@@ -784,9 +790,10 @@ void Job::build_plan(bool pairs) {
   // ones ask: the driver's memory query waits on locks shared with other
   // processes of the machine and took up to 90 ms here (a whole 4x4 chi 4
   // solve: 4.2 ms without it, 4.3 to 30 ms on average with it).
+  const auto slot_bytes = [&](const Unit& U) { return align_elems(site_elems(U.site)) * (U.f64 ? esz : wsz); };
   size_t slots = 0, whole = 0;
   for (const Unit& U : units) {
-    const size_t site_b = align_elems(site_elems(U.site)) * wsz;
+    const size_t site_b = slot_bytes(U);
     slots += (size_t)U.nbuf * site_b;
     whole += (size_t)(U.nbuf + 1) * site_b;
   }
@@ -802,7 +809,7 @@ void Job::build_plan(bool pairs) {
     int last_site = -1;
     for (size_t i = 0; i < units.size(); ++i) {
       const Unit& U = units[i];
-      const size_t site_b = align_elems(site_elems(U.site)) * wsz;
+      const size_t site_b = slot_bytes(U);
       const size_t add = (size_t)U.nbuf * site_b + (U.site == last_site ? 0 : site_b);
       if (waves.empty() || (budget && bytes + add > budget && !waves.back().empty())) {
         waves.emplace_back();
@@ -814,26 +821,25 @@ void Job::build_plan(bool pairs) {
       last_site = U.site;
     }
   }
-  // 3. slot buffers: a wave's units side by side, every wave at offset 0
+  // 3. slot buffers: a wave's units side by side, every wave at byte 0
   std::vector<size_t> unit_base(units.size(), 0);
   size_t scratch = 0;
   for (auto& w : waves) {
     size_t o = 0;
     for (int ui : w) {
       unit_base[ui] = o;
-      o += (size_t)units[ui].nbuf * align_elems(site_elems(units[ui].site));
+      o += (size_t)units[ui].nbuf * slot_bytes(units[ui]);
     }
     scratch = std::max(scratch, o);
   }
   {
     TNBP_TRACE_SCOPE("sweep.build_plan.scratch_alloc");
-    ws_scratch.ensure(std::max<size_t>(scratch, 32) * wsz, stream);
+    ws_scratch.ensure(std::max<size_t>(scratch, 32 * wsz), stream);
   }
   auto slot_ptr = [&](int ui, int slot) -> void* {
     const Unit& U = units[ui];
-    if (slot < 0) return sweep_vptr(U.site);
-    return static_cast<char*>(ws_scratch.p) +
-           (unit_base[ui] + (size_t)U.buf_of_slot.at(slot) * align_elems(site_elems(U.site))) * wsz;
+    if (slot < 0) return U.f64 ? vptr(U.site) : sweep_vptr(U.site);
+    return static_cast<char*>(ws_scratch.p) + unit_base[ui] + (size_t)U.buf_of_slot.at(slot) * slot_bytes(U);
   };
   // 4. tasks
   plan.flops = 0.0;
@@ -876,6 +882,7 @@ void Job::build_plan(bool pairs) {
           lt.mat = mptr(par, g.in_msg(op.site, op.leg));
           lt.L = L; lt.R = R; lt.Din = sh[op.leg]; lt.Dout = sh[op.leg];
           set_leg_divisors(lt);
+          lt.f64 = U.f64;
           lt.block_begin = 0;  // assigned when a batch is built
           W.levels[op.level].tasks[par].push_back(lt);
         }
@@ -883,7 +890,8 @@ void Job::build_plan(bool pairs) {
       for (int t : U.targets) {
         GramTask g1;
         g1.A = slot_ptr(ui, result[U.site][t]);
-        g1.B = sweep_vptr(U.site);
+        g1.B = slot_ptr(ui, -1);
+        g1.f64 = U.f64;
         long long L = 1, M = 1;
         for (int k = 0; k < t; ++k) L *= sh[k];
         for (size_t k = t + 1; k < sh.size(); ++k) M *= sh[k];
@@ -997,7 +1005,8 @@ void Job::build_plan(bool pairs) {
     const int gs = (int)g.legs[s].size();
     for (int par = 0; par < 2; ++par) {
       SiteTask st{};
-      st.V = sweep_vptr(s);
+      st.f64 = prec == TNBP_C128 || (loop && prec == TNBP_MIXED);
+      st.V = st.f64 ? vptr(s) : sweep_vptr(s);
       st.g = gs;
       st.d = pd[s];
       st.n = (int)site_elems(s);
@@ -1036,7 +1045,7 @@ void Job::build_plan(bool pairs) {
       plan.msg[par].push_back(m);
     }
   }
-  plan.pairs = pairs;
+  plan.loop = loop;
   plan.valid = true;
   static std::atomic<uint64_t> serials{0};
   plan_serial = ++serials;
@@ -1105,20 +1114,20 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
   // above on the CUDA cores; complex128 tasks on the FP64 tensor kernel,
   // whatever else shares the batch.  A request's rounding therefore does not
   // depend on what it is batched with.
-  const bool reduced = !entries.empty() && reduced_sweeps(entries[0].job->prec);
-  const bool tc_ok = reduced && tcgen05_enabled();
-  {
+  const bool tc_ok = tcgen05_enabled();
+  for (const int f64 : {0, 1}) {
     // small sites: one CTA per message, on chip
     std::vector<SiteTask> sts;
     size_t smem = 0;
     int degree = 1;
     for (auto& e : entries)
       for (const SiteTask& st : e.job->plan.site[e.parity]) {
+        if (st.f64 != f64) continue;
         sts.push_back(st);
         smem = std::max(smem, site_sweep_smem_bytes(st.D, st.g, st.d));
         degree = std::max(degree, st.g);
       }
-    add(SweepLaunch::SITE, sts, {}, degree, (int)smem);
+    add(f64 ? SweepLaunch::SITE_F64 : SweepLaunch::SITE, sts, {}, degree, (int)smem);
   }
   for (size_t w = 0; w < nw; ++w) {
     {
@@ -1134,15 +1143,21 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
     for (auto& e : entries)
       if (w < e.job->plan.waves.size()) nlev = std::max(nlev, e.job->plan.waves[w].levels.size());
     for (size_t lv = 0; lv < nlev; ++lv) {
-      std::vector<LegTask> t, t2, t3, t4;
-      std::vector<long long> beg, b2, b3, b4;
-      long long nb = 0, nb2 = 0, nb3 = 0, nb4 = 0;
-      int maxdin = 1;
+      std::vector<LegTask> t, t2, t3, t4, t5;
+      std::vector<long long> beg, b2, b3, b4, b5;
+      long long nb = 0, nb2 = 0, nb3 = 0, nb4 = 0, nb5 = 0;
+      int maxdin = 1, maxdin5 = 1;
       for (auto& e : entries) {
         const auto& P = e.job->plan;
         if (w >= P.waves.size() || lv >= P.waves[w].levels.size()) continue;
         for (LegTask lt : P.waves[w].levels[lv].tasks[e.parity]) {
-          if (tc_ok && bulk_leg_enabled() && tc::bulk_mode(lt.L, lt.Din, lt.Dout) != 0) {
+          if (lt.f64) {
+            lt.block_begin = nb5;
+            b5.push_back(nb5);
+            nb5 += dm::leg_tiles(lt.L, lt.R);
+            maxdin5 = std::max(maxdin5, lt.Din);
+            t5.push_back(lt);
+          } else if (tc_ok && bulk_leg_enabled() && tc::bulk_mode(lt.L, lt.Din, lt.Dout) != 0) {
             lt.block_begin = nb3;
             b3.push_back(nb3);
             nb3 += (lt.L * lt.R + tc::kTcRows - 1) / tc::kTcRows;
@@ -1160,7 +1175,7 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
           } else {
             lt.block_begin = nb;
             beg.push_back(nb);
-            nb += reduced ? (lt.L * lt.R + kRowTile - 1) / kRowTile : dm::leg_tiles(lt.L, lt.R);
+            nb += (lt.L * lt.R + kRowTile - 1) / kRowTile;
             maxdin = std::max(maxdin, lt.Din);
             t.push_back(lt);
           }
@@ -1170,17 +1185,19 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
       add(SweepLaunch::LEG_T64, t4, b4, nb4, 0);
       add(SweepLaunch::LEG_TC, t2, b2, nb2, 0);
       add(SweepLaunch::LEG_CORE, t, beg, nb, maxdin);
+      add(SweepLaunch::LEG_F64, t5, b5, nb5, maxdin5);
     }
     // Gram tasks: the fused absorption + Gram kernel, then per task the
-    // tcgen05 kernels (one CTA per chunk) for the complex64 sweeps with C <=
-    // 64, else the CUDA-core kernel; then the wave's messages are finalized
-    std::vector<GramTask> gt, gt2, gt3;
-    std::vector<long long> gb, gb2, gb3, lb;
+    // tcgen05 kernels (one CTA per chunk) for complex64 with C <= 64, the
+    // FP64 tensor kernel for complex128, else the CUDA-core kernel; then the
+    // wave's messages are finalized
+    std::vector<GramTask> gt, gt2, gt3, gt4;
+    std::vector<long long> gb, gb2, gb3, gb4, lb;
     std::vector<LegGramTask> lt;
     std::vector<LegPairTask> pt[2];  // 4 and 8 planes per tile
     std::vector<long long> pb[2];
     std::vector<MsgTask> mt;
-    long long nb = 0, nb2 = 0, nb3 = 0, nlb = 0, npb[2] = {0, 0};
+    long long nb = 0, nb2 = 0, nb3 = 0, nb4 = 0, nlb = 0, npb[2] = {0, 0};
     for (auto& e : entries) {
       const auto& P = e.job->plan;
       if (w >= P.waves.size()) continue;
@@ -1197,7 +1214,12 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
       for (int mi : P.waves[w].msgs) mt.push_back(P.msg[e.parity][mi]);
       for (int gi : P.waves[w].grams) {
         GramTask g1 = P.gram[gi];
-        if (tc_ok && tc::gram_tc_ok(g1.C, g1.P)) {
+        if (g1.f64) {
+          g1.block_begin = nb4;
+          gb4.push_back(nb4);
+          nb4 += P.gram_blocks[gi];
+          gt4.push_back(g1);
+        } else if (tc_ok && tc::gram_tc_ok(g1.C, g1.P)) {
           g1.block_begin = nb2;
           gb2.push_back(nb2);
           nb2 += g1.nchunk;
@@ -1220,6 +1242,7 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
     add(SweepLaunch::GRAM_TC, gt2, gb2, nb2, 0);
     add(SweepLaunch::GRAM_T64, gt3, gb3, nb3, 0);
     add(SweepLaunch::GRAM_CORE, gt, gb, nb, 0);
+    add(SweepLaunch::GRAM_F64, gt4, gb4, nb4, 0);
     add(SweepLaunch::MSG, mt, {}, (long long)mt.size(), 0);
   }
   // one condition per job
@@ -1313,13 +1336,18 @@ static int launch_batch_t(const SweepBatch& b, cudaStream_t stream) {
       }
       case SweepLaunch::LEG_CORE: {
         if (L.max_din > 128) throw Error(TNBP_EUNSUPPORTED, "bond dimension above 128 during BP");
-        if constexpr (sizeof(R) == 8)
-          launch_leg_f64(static_cast<const LegTask*>(tasks), begins, L.ntask, L.nblocks, L.max_din, stream);
-        else
+        if constexpr (sizeof(R) == 4)
           k_leg_apply<R, MR><<<(unsigned)L.nblocks, kThreads, leg_smem<R>(L.max_din), stream>>>(
               static_cast<const LegTask*>(tasks), begins, L.ntask, L.max_din);
         break;
       }
+      case SweepLaunch::LEG_F64:
+        if (L.max_din > 128) throw Error(TNBP_EUNSUPPORTED, "bond dimension above 128 during BP");
+        launch_leg_f64(static_cast<const LegTask*>(tasks), begins, L.ntask, L.nblocks, L.max_din, stream);
+        break;
+      case SweepLaunch::GRAM_F64:
+        launch_gram_f64(static_cast<const GramTask*>(tasks), begins, L.ntask, L.nblocks, stream);
+        break;
       case SweepLaunch::GRAM_TC:
         k_gram_tc<<<(unsigned)L.nblocks, 256, tc::gram_smem_bytes(), stream>>>(
             static_cast<const GramTask*>(tasks), begins, L.ntask);
@@ -1345,16 +1373,18 @@ static int launch_batch_t(const SweepBatch& b, cudaStream_t stream) {
         break;
       }
       case SweepLaunch::GRAM_CORE:
-        if constexpr (sizeof(R) == 8)
-          launch_gram_f64(static_cast<const GramTask*>(tasks), begins, L.ntask, L.nblocks, stream);
-        else
+        if constexpr (sizeof(R) == 4)
           k_gram<R><<<(unsigned)L.nblocks, kThreads, 0, stream>>>(static_cast<const GramTask*>(tasks), begins, L.ntask);
         break;
       case SweepLaunch::MSG:
         k_msg_finalize<R, MR><<<L.ntask, kFinalizeThreads, 0, stream>>>(static_cast<const MsgTask*>(tasks));
         break;
       case SweepLaunch::SITE:  // max_din holds the launch's shared memory bytes, nblocks the largest degree
-        k_site_sweep<R, MR><<<dim3((unsigned)L.ntask, (unsigned)L.nblocks), kThreads, (size_t)L.max_din, stream>>>(static_cast<const SiteTask*>(tasks));
+        if constexpr (sizeof(R) == 4)
+          k_site_sweep<R, MR><<<dim3((unsigned)L.ntask, (unsigned)L.nblocks), kThreads, (size_t)L.max_din, stream>>>(static_cast<const SiteTask*>(tasks));
+        break;
+      case SweepLaunch::SITE_F64:
+        k_site_sweep<double, double><<<dim3((unsigned)L.ntask, (unsigned)L.nblocks), kThreads, (size_t)L.max_din, stream>>>(static_cast<const SiteTask*>(tasks));
         break;
       case SweepLaunch::SUM:
         k_segmented_sum<<<L.ntask, kThreads, 0, stream>>>(static_cast<const SumTask*>(tasks));
@@ -1407,6 +1437,7 @@ void prepare_kernels(int prec) {
     tc_attr<float>();
   } else {
     leg_apply_attr<float, double>();
+    leg_apply_attr<double, double>();  // the sites of site_f64
     tc_attr<double>();
   }
 }
@@ -1471,6 +1502,24 @@ bool site_sweep_enabled() {
     return !(e && e[0] == '0');
   }();
   return on;
+}
+
+// The mixed path's loops sweep sites whose bond dimensions are all at most 8
+// (and the on-chip ones of site_whole, whose arithmetic is FP64 anyway) in
+// complex128, from V instead of its complex64 copy.  Circuits build such
+// bonds, and their observables' terms nearly cancel, so that the messages'
+// rounding comes back enlarged: over 24 random circuits up to 10x10 with 12
+// layers and 48 random terms the total was off by up to 2e-5 of itself with
+// these sites in pairs of legs (median 4e-7), 6e-6 leg by leg (4e-7), 1.5e-6
+// with the on-chip ones alone still reading the copy, 5e-8 (output rounding)
+// like this.  At these sizes a sweep is launches and latency: one sweep of a
+// 10x10 lattice's loop takes 89 us at D = 6 (114 in pairs of legs, 122 leg by
+// leg), 133 at D = 8 (162, 179) and 186 at D = 9 (230); at D = 12 FP64 takes
+// 354 and pairs 320, so the line could lie up to 11, but nothing above 8 needs
+// it.
+bool Job::site_f64(int s) const {
+  const auto sh = site_shape(s);
+  return prec == TNBP_MIXED && *std::max_element(sh.begin(), sh.end() - 1) <= kMixedF64Dim;
 }
 
 bool Job::site_whole(int s) const {

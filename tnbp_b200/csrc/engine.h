@@ -87,7 +87,7 @@ struct WaveHost {
 // One kernel launch of a sweep batch; its task arrays live in the batch's
 // arena at the given byte offsets.
 struct SweepLaunch {
-  enum Kind { LEG_BULK, LEG_T64, LEG_TC, LEG_CORE, GRAM_TC, GRAM_T64, GRAM_CORE, LEG_GRAM, PAIR_ABSORB, PAIR_GRAM, MSG, SUM, SITE };
+  enum Kind { LEG_BULK, LEG_T64, LEG_TC, LEG_CORE, GRAM_TC, GRAM_T64, GRAM_CORE, LEG_GRAM, PAIR_ABSORB, PAIR_GRAM, LEG_F64, GRAM_F64, MSG, SUM, SITE, SITE_F64 };
   int kind;
   size_t tasks_off, begins_off;
   int ntask;
@@ -118,8 +118,8 @@ struct SweepBatch {
 
 struct SweepPlan {
   bool valid = false;
-  bool pairs = false;     // degree-4 sites by pairs of legs, where they can be
-  bool pairable = false;  // some can
+  bool loop = false;      // made for the loop's sweeps
+  bool varies = false;    // single sweeps take some sites another way
   DevBuf partial, dist;
   std::vector<WaveHost> waves;
   std::vector<GramTask> gram;
@@ -144,6 +144,7 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
 int launch_batch(const SweepBatch& b, int prec, cudaStream_t stream);
 void note_launch(int n = 1);
 void keep_pool_memory();
+constexpr int kMixedF64Dim = 8;  // see Job::site_f64
 constexpr double kC64TolFloor = 1e-7;
 constexpr double kC64GrowthGate = 1e-5;
 double effective_tol(int prec, double tol);
@@ -244,6 +245,7 @@ struct Job {
   Job(const int32_t* e, int64_t n, const int32_t* pdims, int precision, cudaStream_t s, uint64_t budget);
   ~Job();
   std::vector<int> site_shape(int s) const;
+  bool site_f64(int s) const;    // swept in complex128 by the mixed path's loops
   bool site_whole(int s) const;  // swept whole on chip by k_site_sweep
   size_t site_elems(int s) const;
   void layout();
@@ -256,9 +258,9 @@ struct Job {
   void sync_shadow();
   void* mptr(int arena, int m) const;
   void destroy_graphs();
-  void build_plan(bool pairs = true);
-  // A plan for the loop's sweeps (pairs) or for single sweeps.
-  void ensure_plan(bool pairs);
+  void build_plan(bool loop = true);
+  // A plan for the loop's sweeps or for single sweeps.
+  void ensure_plan(bool loop);
   size_t scratch_limit() const;
   void run_sweep(int par);
   double read_cond();

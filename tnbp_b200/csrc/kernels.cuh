@@ -55,6 +55,7 @@ struct LegTask {
   long long block_begin;  // exclusive prefix of row tiles over tasks
   FastDiv div_l;          // by L: the CUDA-core kernel's row split q = l + L r
   FastDiv div_din;        // by Din
+  int f64 = 0;            // complex128 operands
 };
 inline void set_leg_divisors(LegTask& t) {
   t.div_l = make_fastdiv((uint32_t)t.L);
@@ -157,6 +158,7 @@ struct GramTask {
   int nchunk;
   double2* partial;       // [nchunk][C*C], N[c + C*c']
   long long block_begin;  // exclusive prefix of nchunk*ctiles*ctiles
+  int f64 = 0;            // complex128 operands
 };
 
 template <typename R>
@@ -280,6 +282,7 @@ struct SiteTask {
   double* dist[kMaxLegs];      // || new/|new| - old/|old| ||_F of leg k
   int D[kMaxLegs];
   int g, d, n;                 // degree, physical dim, d prod D
+  int f64 = 0;                 // V in complex128
 };
 
 // Shared memory of one site: V and two buffers of n complex FP64 values, the

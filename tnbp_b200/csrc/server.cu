@@ -87,18 +87,21 @@ uint64_t footprint_estimate(const std::vector<std::pair<int, int>>& edges, const
   std::map<int, size_t> pos;
   for (size_t i = 0; i < sites.size(); ++i) pos[sites[i]] = i;
   std::vector<double> n(sites.size(), 2.0);  // elements of each site tensor
+  std::vector<double> most(sites.size(), 1.0);  // its largest bond
   std::vector<int> deg(sites.size(), 0);
   for (size_t e = 0; e < ne; ++e)
     for (int v : {edges[e].first, edges[e].second}) {
       n[pos[v]] *= D[e];
+      most[pos[v]] = std::max(most[pos[v]], D[e]);
       ++deg[pos[v]];
     }
   double bytes = 0.0, slots_all = 0.0, unit_max = 0.0, chain_all = 0.0;
   for (size_t i = 0; i < sites.size(); ++i) {
     bytes += n[i] * (2.0 * esz + shadow);  // V, spare, sweep copy
     chain_all += n[i] * esz;
-    slots_all += n[i] * wsz * sweep_slots(deg[i]);
-    unit_max = std::max(unit_max, n[i] * wsz * std::max(1, deg[i]));
+    const double slot = n[i] * (most[i] <= kMixedF64Dim ? esz : wsz);
+    slots_all += slot * sweep_slots(deg[i]);
+    unit_max = std::max(unit_max, slot * std::max(1, deg[i]));
   }
   bytes += 2.0 * std::min(chain_all, (double)chain_cap_bytes());
   // sweep scratch: one wave's units at a time (a wave stays within the wave

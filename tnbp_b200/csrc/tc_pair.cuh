@@ -14,11 +14,11 @@
 // HBM and launch tails to what lies between the hand-overs of a tile: shared
 // memory (operand stores and MMA reads, about 6000 cycles per tile at D =
 // 32), conversions, FP64 additions and waits.  So two groups of warps, one
-// per target, share the tiles but nothing else and fill each other's gaps
-// (cycles per tile with one group that took the targets in turn: 12200 at D =
-// 32, 9850 at 24, 10600 at 16; now 11550, 8950, 8900).  One 8x8 sweep at
-// D = 32 (36 degree-4 sites): 3.96 ms in the separate kernels, 1.52 ms here;
-// 6x6 at D = 16: 0.17 -> 0.09 ms.
+// per target, share the tiles but nothing else and fill each other's gaps (5 %
+// of the tile's cycles at D = 32, 16 % at 16, against one group that takes the
+// targets in turn).  One sweep of an 8x8 lattice's loop at D = 32 (36 degree-4
+// sites): 3.96 ms in the separate kernels, 1.85 ms here; 6x6 at D = 16: 0.17
+// -> 0.11 ms, at D = 24 0.46 ms.
 //
 // A tile is P planes (P Dx, P Dy <= 128 rows): raw complex64 planes arrive by
 // cp.async, two tiles in flight, placed as PairLayout says.  Per target (say
@@ -32,7 +32,17 @@
 //      y at a time: rows [re_hi; im_hi; re_lo; im_lo] x 32 of 8 P contraction
 //      columns (o, y); one M = 128, N = 128 MMA per 8 columns gives all four
 //      hi/lo products
-//   3. the tile's FP32 Gram is added to FP64 registers.
+//   3. after 64 columns the FP32 Gram is added to FP64 registers, the cross
+//      products apart from the main ones.
+// Step 3 costs a fifth of the kernel (1.50 ms at D = 32, 0.089 at 16, 0.34 at
+// 24 with one FP32 sum per tile, cross products added to it in FP32), but so
+// these sums are no coarser than k_gram_tc's: the tensor core truncates as it
+// accumulates, so that the error grows with the run and is of one sign.
+// Messages of a degree-4 site against 64 bits, root mean square over 12 seeds
+// with decaying bonds, leg by leg / one sum per tile / like this, in 1e-8:
+// 18.1 / 13.2 / 11.5 at D = 32, 12.6 / 14.7 / 11.0 at 16, 10.1 / 11.0 / 9.9 at
+// 12; the mixed 16x16 chi 16 solve takes 62 sweeps instead of 67 and its |dE|
+// is 7e-8 instead of 8.9e-7.
 // A chunk of tiles ends in one FP64 partial per target, reduced by
 // k_msg_finalize in a fixed order.
 //
@@ -359,6 +369,7 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
   // do not wait for this tile's N).
   constexpr uint32_t kBlk = P == 4 ? 32 : 16, kColP = 4 * kBlk, kColN = P == 4 ? 0 : 8 * kBlk;
   constexpr bool kAhead = P != 4;
+  constexpr uint32_t kStages = P == 4 ? 2 : 1;  // of 8 P contraction columns: N starts afresh after 64
 
   // A bounded wait by a whole warp; false (for the whole warp) when it or
   // any other thread of the CTA gave up.
@@ -393,7 +404,9 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
     PairRow<P> pr_row;
 
     // N of this row: columns 8 i + 4 g + k (those whose place this warp's
-    // part of the next A takes)
+    // part of the next A takes), v against the hi rows of V, u against the lo
+    // ones; of a hi row u is 2^-11 of v and they meet in FP64, a lo row's are
+    // both that small
     auto drain = [&]() {
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
@@ -404,8 +417,13 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
         tmem_ld4_async(c + 64, u);
         tmem_ld4_async(c + 72, u + 4);
         tmem_ld_wait16(v, v + 4, u, u + 4);
+        if ((w8 & 3) < 2) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[8 * h + i] += (double)(v[i] + u[i]);
+          for (int i = 0; i < 8; ++i) acc[8 * h + i] += (double)v[i] + (double)u[i];
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[8 * h + i] += (double)(v[i] + u[i]);
+        }
       }
     };
     auto read4 = [&](const float2* t, uint32_t j, float4& re, float4& im) {
@@ -490,6 +508,7 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
         put_op(op, re, im);
         put_op(op + kOp, vr, vi);
       }
+      if (s > 0 && s % kStages == 0) drain();
       publish(bar_ready + 8u * target);
       return true;
     };
@@ -625,7 +644,7 @@ __device__ __forceinline__ void pair_gram(const LegPairTask* __restrict__ tasks,
             if (elect_one()) {
 #pragma unroll
               for (uint32_t s = 0; s < P; ++s)
-                mma_tf32(base + kColN, da + pair_group(P) / 8 * s, db + pair_group(P) / 8 * s, idesc_tf32(128, 128), st + s);
+                mma_tf32(base + kColN, da + pair_group(P) / 8 * s, db + pair_group(P) / 8 * s, idesc_tf32(128, 128), st % kStages + s);
               mma_commit(bar_done + 8u * target);
             }
             __syncwarp();

@@ -371,8 +371,7 @@ int tnbp_load_state(tnbp_job* job, const char* path) {
     J.put_complex(J.M[0], hm.data(), J.m_elems, 0);
     J.cur = 0;
     J.shadow_dirty = true;
-    J.destroy_graphs();
-    J.plan = tnbp::SweepPlan();
+    J.drop_plans();
   });
 }
 
@@ -492,8 +491,7 @@ int tnbp_upload_message(tnbp_job* job, int64_t m, int32_t dim, const double* dat
         if (J.dim[k % ne] == odim[k % ne])
           J.put_complex(J.M[0], keepM.data() + 2 * omoff[k], (size_t)odim[k % ne] * odim[k % ne], J.moff[k]);
       J.cur = 0;
-      J.destroy_graphs();
-      J.plan = tnbp::SweepPlan();
+      J.drop_plans();
     }
     J.put_complex(J.M[J.cur], data, (size_t)dim * dim, J.moff[m]);
   });

@@ -242,11 +242,10 @@ Job::Job(const int32_t* e, int64_t n, const int32_t* pdims, int precision, cudaS
 }
 
 Job::~Job() {
-  destroy_graphs();
   cudaStreamSynchronize(stream);
   V.release(); M[0].release(); M[1].release(); V32.release();
   ws_scratch.release(); ws_chain[0].release(); ws_chain[1].release(); Vspare.release();
-  plan = SweepPlan();
+  drop_plans();
   if (host_scalar) pinned_slot_put(host_scalar);
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
@@ -286,6 +285,7 @@ void Job::layout() {
 void Job::put_complex(DevBuf& dst, const double* src, size_t n, size_t elem_off) {
   if (n == 0) return;
   if (&dst == &V) shadow_dirty = true;
+  if (&dst == &M[0] || &dst == &M[1]) loop_messages = false;
   if (sprec == TNBP_C128) {
     CK(cudaMemcpyAsync(static_cast<char*>(dst.p) + elem_off * 16, src, n * 16, cudaMemcpyHostToDevice, stream));
     CK(cudaStreamSynchronize(stream));
@@ -311,7 +311,7 @@ void Job::get_complex(const DevBuf& src, double* dst, size_t n, size_t elem_off)
 
 uint64_t Job::device_bytes() const {
   return V.bytes + M[0].bytes + M[1].bytes + V32.bytes + ws_scratch.bytes + ws_chain[0].bytes +
-         ws_chain[1].bytes + Vspare.bytes + plan.bytes();
+         ws_chain[1].bytes + Vspare.bytes + plan.bytes() + idle.bytes();
 }
 void Job::check_budget() const {
   if (budget && device_bytes() > budget)
@@ -326,14 +326,11 @@ void* Job::sweep_vptr(int s) const {
 
 // TNBP_MIXED: round the complex128 site tensors to the complex64 copy that
 // the sweeps read (the copy only grows).  A re-allocated copy invalidates the
-// sweep plan (its tasks and graphs hold the old addresses).
+// sweep plans (their tasks and graphs hold the old addresses).
 void Job::sync_shadow() {
   if (prec != TNBP_MIXED || !shadow_dirty) return;
   TNBP_TRACE_SCOPE("sweep.sync_shadow");
-  if (V32.ensure(v_elems * 8, stream)) {
-    destroy_graphs();
-    plan = SweepPlan();
-  }
+  if (V32.ensure(v_elems * 8, stream)) drop_plans();
   const unsigned grid = (unsigned)std::min<size_t>((v_elems + 255) / 256, (size_t)8 * num_sms());
   k_narrow<<<grid, 256, 0, stream>>>(static_cast<const double2*>(V.p), static_cast<float2*>(V32.p), v_elems);
   CK(cudaGetLastError());
@@ -342,9 +339,9 @@ void Job::sync_shadow() {
 }
 void* Job::mptr(int arena, int m) const { return static_cast<char*>(M[arena].p) + moff[m] * esz; }
 
-void Job::destroy_graphs() {
-  plan.single[0].reset_graph();
-  plan.single[1].reset_graph();
+void Job::drop_plans() {
+  plan = SweepPlan();
+  idle = SweepPlan();
 }
 
 void SweepBatch::reset_graph() {
@@ -684,9 +681,7 @@ void Job::autotune_waves() {
   size_t best_mb = wave_budget_bytes() >> 20;
   for (size_t mb : kWaveCandidatesMb) {
     wave_budget = mb << 20;
-    destroy_graphs();
-    plan = SweepPlan();
-    build_plan();
+    build_plan(true);
     run_sweep(cur);  // warm-up (and graph capture); the state is unchanged
     double ms = 0.0;
     for (int rep = 0; rep < 2; ++rep) {
@@ -707,8 +702,7 @@ void Job::autotune_waves() {
     if (ms < 0.97 * best_ms) { best_ms = ms; best_mb = mb; }
   }
   wave_budget = best_mb << 20;
-  destroy_graphs();
-  plan = SweepPlan();
+  build_plan(true);
   TuneTable& T = tune_table();
   std::lock_guard<std::mutex> lk(T.mu);
   device_table(dev)[key] = best_mb;
@@ -731,16 +725,19 @@ void Job::autotune_waves() {
 // from any fixed point, where loopy BP amplifies rounding (random states: 600
 // to 1000 times in four sweeps).  Their results do not depend on how fast a
 // loop is.  36 sites at D = 32, d = 2, per sweep: 5.8 ms leg by leg, 2.4 ms in
-// pairs.
+// pairs.  A program that changes between the two keeps both plans and their
+// graphs (building one takes the host longer than most sweeps), as long as
+// the shared scratch does not move and the budget holds both.
 void Job::ensure_plan(bool loop) {
-  if (!plan.valid || (plan.varies && plan.loop != loop)) build_plan(loop);
+  if (plan.valid && (!plan.varies || plan.loop == loop)) return;
+  if (plan.valid) std::swap(plan, idle);
+  if (!plan.valid || plan.loop != loop) build_plan(loop);
 }
 
 void Job::build_plan(bool loop) {
   TNBP_TRACE_SCOPE("sweep.build_plan");
   {
     TNBP_TRACE_SCOPE("sweep.build_plan.release");
-    destroy_graphs();
     plan = SweepPlan();
   }
   const int ns = (int)g.labels.size();
@@ -834,7 +831,9 @@ void Job::build_plan(bool loop) {
   }
   {
     TNBP_TRACE_SCOPE("sweep.build_plan.scratch_alloc");
-    ws_scratch.ensure(std::max<size_t>(scratch, 32 * wsz), stream);
+    const size_t need = std::max<size_t>(scratch, 32 * wsz);
+    if (ws_scratch.bytes < need) idle = SweepPlan();  // it holds the old address
+    ws_scratch.ensure(need, stream);
   }
   auto slot_ptr = [&](int ui, int slot) -> void* {
     const Unit& U = units[ui];
@@ -997,7 +996,13 @@ void Job::build_plan(bool loop) {
   }
   // Gram partials are finalized at the end of their wave, so one wave's
   // worth of partials is enough
-  plan.partial.alloc(max_part * sizeof(double2), stream);
+  try {
+    plan.partial.alloc(max_part * sizeof(double2), stream);
+  } catch (const Error&) {
+    if (!idle.valid) throw;
+    idle = SweepPlan();
+    plan.partial.alloc(max_part * sizeof(double2), stream);
+  }
   plan.dist.alloc(std::max<size_t>(2 * ne, 1) * sizeof(double), stream);
   for (int par = 0; par < 2; ++par) plan.site[par].clear();
   for (int s : small_sites) {
@@ -1048,11 +1053,12 @@ void Job::build_plan(bool loop) {
   plan.loop = loop;
   plan.valid = true;
   static std::atomic<uint64_t> serials{0};
-  plan_serial = ++serials;
+  plan.serial = ++serials;
   // the per-job launch sequences (plan.single) are built on first use: a
   // served job only ever runs inside batches.  Every allocation above is
   // stream-ordered and every upload is staged before it returns, so no
   // synchronization is needed here.
+  if (budget && device_bytes() > budget) idle = SweepPlan();
   check_budget();
 }
 
@@ -1065,10 +1071,7 @@ void build_batch(const std::vector<BatchEntry>& entries, SweepBatch& b, cudaStre
   b.reset_graph();
   b.launches.clear();
   size_t nw = 0;
-  for (auto& e : entries) {
-    if (!e.job->plan.valid) e.job->build_plan();
-    nw = std::max(nw, e.job->plan.waves.size());
-  }
+  for (auto& e : entries) nw = std::max(nw, e.job->plan.waves.size());
   std::vector<unsigned char> host;
   auto put = [&](const void* p, size_t bytes) -> size_t {
     const size_t off = (host.size() + 255) & ~size_t(255);
@@ -1551,9 +1554,7 @@ void check_tc_error(cudaStream_t stream) {
 // capture) than the sweeps themselves.
 constexpr int kEagerSweeps = 2;
 
-void Job::run_sweep(int par) {
-  sync_shadow();
-  if (!plan.valid) build_plan();
+void Job::run_sweep(int par) {  // of a valid plan (sync_shadow, ensure_plan)
   SweepBatch& b = plan.single[par];
   if (b.launches.empty()) build_batch({{this, par}}, b, stream);
   if (!b.graph && b.uses < kEagerSweeps) {
@@ -1610,13 +1611,16 @@ void Job::bp_sweep() {
   ensure_plan(false);
   run_sweep(cur);
   cur = 1 - cur;
+  loop_messages = false;
   CK(cudaStreamSynchronize(stream));
   if (reduced_sweeps(prec)) check_tc_error(stream);
 }
 
+// By the sweep that made the messages: after a loop this is the condition
+// that the loop ended with, to the bit.
 double Job::bp_condition() {
   sync_shadow();
-  ensure_plan(false);
+  ensure_plan(loop_messages);
   run_sweep(cur);  // writes the other arena; state (cur) unchanged
   return read_cond();
 }
@@ -1653,6 +1657,7 @@ void Job::bp_run(double tol_in, int max_iter, int* iters, double* cond) {
   autotune_waves();
   run_sweep(cur);
   cur = 1 - cur;
+  loop_messages = true;
   *iters = 1;
   double prev = INFINITY;
   while (true) {
@@ -1689,9 +1694,8 @@ void Job::absorb_tpo(const Tpo& tpo) {
   nV.ensure(v_elems * esz, stream);
   nM0.alloc(m_elems * esz, stream);
   nM1.alloc(m_elems * esz, stream);
-  plan.valid = false;
-  destroy_graphs();
-  plan = SweepPlan();  // it holds the old addresses
+  drop_plans();  // they hold the old addresses
+  loop_messages = false;
   // the mixed path's complex64 copy is written along if it fits now, else
   // before the first sweep (sync_shadow)
   bool along = prec == TNBP_MIXED &&
@@ -1886,6 +1890,7 @@ static void launch_truncation(const TruncTask* tasks, int ne, int max_d, int chi
 void Job::truncate(int chi_max, double sv_min, int32_t* dims_out, double* err_out) {
   TNBP_TRACE_SCOPE("truncate");
   shadow_dirty = true;
+  idle = SweepPlan();  // its bonds end here
   if (chi_max < 1) throw Error(TNBP_EINVAL, "chi_max must be >= 1");
   const int ns = (int)g.labels.size();
   const int ne = (int)g.edges.size();
@@ -1987,9 +1992,8 @@ void Job::truncate(int chi_max, double sv_min, int32_t* dims_out, double* err_ou
   std::swap(M[0], nM0);
   std::swap(M[1], nM1);
   cur = 0;
-  plan.valid = false;
-  destroy_graphs();
-  plan = SweepPlan();
+  loop_messages = false;
+  drop_plans();
   // no synchronization: the kept dims and errors are already on the host,
   // the buffers above are freed in stream order and the uploads were staged
   // before they returned, so the host goes on while the projectors run

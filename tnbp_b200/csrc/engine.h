@@ -131,6 +131,7 @@ struct SweepPlan {
   std::vector<SiteTask> site[2];       // sites swept whole on chip (k_site_sweep), per parity
   SweepBatch single[2];
   double flops = 0.0, bytes_alg = 0.0;
+  uint64_t serial = 0;    // unique per build (keys of the server's sweep graphs)
   SweepPlan() = default;
   SweepPlan(SweepPlan&&) = default;
   SweepPlan& operator=(SweepPlan&&) = default;
@@ -232,8 +233,9 @@ struct Job {
   DevBuf ws_scratch, ws_chain[2], Vspare;
   int cur = 0;
   int last_par = 0;
-  SweepPlan plan;
-  uint64_t plan_serial = 0;  // unique per plan build (keys of the server's sweep graphs)
+  SweepPlan plan;              // of the last sweep
+  SweepPlan idle;              // the other schedule's, while its addresses hold
+  bool loop_messages = false;  // the messages come from a loop's sweep
   size_t wave_budget = 0;    // wave byte budget of the next plan (0: one wave)
   size_t scratch_cap = 0;    // most sweep-slot bytes a plan may hold (0: from free device memory)
   bool tuning = false;       // the autotuner sets wave_budget itself
@@ -257,9 +259,9 @@ struct Job {
   void* sweep_vptr(int s) const;
   void sync_shadow();
   void* mptr(int arena, int m) const;
-  void destroy_graphs();
-  void build_plan(bool loop = true);
-  // A plan for the loop's sweeps or for single sweeps.
+  void drop_plans();
+  void build_plan(bool loop);
+  // Makes `plan` one for the loop's sweeps or for single sweeps.
   void ensure_plan(bool loop);
   size_t scratch_limit() const;
   void run_sweep(int par);

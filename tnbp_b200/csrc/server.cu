@@ -299,7 +299,7 @@ Server::GroupSweep Server::prepare_group(int gprec, const std::vector<Request*>&
   }
   prepare_kernels(gprec);
   std::vector<uint64_t> key;
-  for (auto& e : entries) key.push_back(2 * e.job->plan_serial + (uint64_t)e.parity);
+  for (auto& e : entries) key.push_back(2 * e.job->plan.serial + (uint64_t)e.parity);
   auto it = sweeps.find(key);
   if (it == sweeps.end()) {
     auto cs = std::make_unique<CachedSweep>();

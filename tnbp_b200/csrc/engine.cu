@@ -1677,25 +1677,41 @@ void Job::bp_run(double tol_in, int max_iter, int* iters, double* cond) {
 // --------------------------------------------------------------- AbsorbTPO
 Tpo::~Tpo() {}
 
+// A call that is refused or runs out of memory leaves the state as it was: V
+// and the messages are replaced at the very end, the layout is put back.
 void Job::absorb_tpo(const Tpo& tpo) {
   TNBP_TRACE_SCOPE("absorb");
   const int ns = (int)g.labels.size();
   const int ne = (int)g.edges.size();
   if ((int)tpo.rank.size() != ne) throw Error(TNBP_EINVAL, "TPO edge count mismatch");
-  std::vector<int> ndim(ne);
-  for (int e = 0; e < ne; ++e) ndim[e] = dim[e] * tpo.rank[e];
+  for (int s = 0; s < ns; ++s) {
+    double n = pd[s];
+    for (int e : g.legs[s]) n *= (double)dim[e] * tpo.rank[e];
+    if (n >= 2147483648.0) throw Error(TNBP_EUNSUPPORTED, "site tensor of 2^31 or more elements");
+  }
   const std::vector<int> odim = dim;
   const std::vector<size_t> ovoff = voff, omoff = moff;
-  // new layout
-  dim = ndim;
-  layout();
   DevBuf nM0, nM1;
   DevBuf& nV = Vspare;
+  // the plans hold the old addresses, and the complex64 copy may be written
+  // or move below
+  drop_plans();
+  shadow_dirty = true;
+  struct Layout {
+    Job& j;
+    const std::vector<int>& odim;
+    bool keep = false;
+    ~Layout() {
+      if (keep) return;
+      j.dim = odim;
+      j.layout();
+    }
+  } layout_guard{*this, odim};
+  for (int e = 0; e < ne; ++e) dim[e] *= tpo.rank[e];
+  layout();
   nV.ensure(v_elems * esz, stream);
   nM0.alloc(m_elems * esz, stream);
   nM1.alloc(m_elems * esz, stream);
-  drop_plans();  // they hold the old addresses
-  loop_messages = false;
   // the mixed path's complex64 copy is written along if it fits now, else
   // before the first sweep (sync_shadow)
   bool along = prec == TNBP_MIXED &&
@@ -1727,7 +1743,6 @@ void Job::absorb_tpo(const Tpo& tpo) {
       t.nv *= t.Dv[k];
       t.ncombo *= t.r[k];
     }
-    if ((long long)site_elems(s) >= (1ll << 31)) throw Error(TNBP_EUNSUPPORTED, "site tensor of 2^31 or more elements");
     t.vblocks = (int)((t.nv + kThreads - 1) / kThreads);
     t.block_begin = nb;
     ab.push_back(nb);
@@ -1762,7 +1777,9 @@ void Job::absorb_tpo(const Tpo& tpo) {
     (k_expand_msgs<float><<<(unsigned)nmb, kThreads, 0, stream>>>(static_cast<MsgExpandTask*>(dmt.p), static_cast<long long*>(dmb.p), (int)mt.size()), note_launch());
   }
   CK(cudaGetLastError());
+  layout_guard.keep = true;
   shadow_dirty = !along;
+  loop_messages = false;
   std::swap(V, nV);
   std::swap(M[0], nM0);
   std::swap(M[1], nM1);

@@ -637,8 +637,11 @@ std::map<std::string, size_t>& device_table(int dev) {
 }
 }  // namespace
 
-// Shape class of a job: precision, largest bond dimension, largest site
-// degree and the site count rounded up to a power of two.
+// Class of a plan: precision, largest bond dimension, largest site degree, the
+// site count rounded up to a power of two, the schedule where loops and single
+// sweeps differ (their slots and kernels do), and the version of the kernels
+// that a table was tuned on (raised with them: a file outlives a build).
+constexpr const char* kTuneVersion = "_k2";
 std::string Job::tune_key() const {
   int maxd = 1, maxg = 0;
   for (int d : dim) maxd = std::max(maxd, d);
@@ -646,7 +649,9 @@ std::string Job::tune_key() const {
   size_t ns = 1;
   while (ns < g.labels.size()) ns <<= 1;
   const char* pn = prec == TNBP_C128 ? "c128" : prec == TNBP_C64 ? "c64" : "mixed";
-  return std::string(pn) + "_D" + std::to_string(maxd) + "_g" + std::to_string(maxg) + "_n" + std::to_string(ns);
+  const char* sched = !plan.varies ? "" : plan.loop ? "_loop" : "_single";
+  return std::string(pn) + "_D" + std::to_string(maxd) + "_g" + std::to_string(maxg) + "_n" + std::to_string(ns) + sched +
+         kTuneVersion;
 }
 
 void Job::choose_wave_budget() {
@@ -739,6 +744,7 @@ void Job::build_plan(bool loop) {
   {
     TNBP_TRACE_SCOPE("sweep.build_plan.release");
     plan = SweepPlan();
+    plan.loop = loop;
   }
   const int ns = (int)g.labels.size();
   const int ne = (int)g.edges.size();
@@ -1050,7 +1056,6 @@ void Job::build_plan(bool loop) {
       plan.msg[par].push_back(m);
     }
   }
-  plan.loop = loop;
   plan.valid = true;
   static std::atomic<uint64_t> serials{0};
   plan.serial = ++serials;

@@ -269,7 +269,7 @@ struct Job {
   void bp_sweep();
   double bp_condition();
   void bp_run(double tol, int max_iter, int* iters, double* cond);
-  std::string tune_key() const;
+  std::string tune_key() const;  // of the plan being built
   void choose_wave_budget();
   void autotune_waves();
   void absorb_tpo(const Tpo& tpo);

@@ -507,13 +507,11 @@ int tnbp_tpo_create(tnbp_job* job, const int32_t* edge_rank, const int64_t* op_o
     t->rank.assign(edge_rank, edge_rank + ne);
     for (int r : t->rank) need(r >= 1, "TPO bond rank must be >= 1");
     t->op_offset.assign(op_offset, op_offset + ns);
-    t->dout.resize(ns);
     int64_t total = 0;
     for (int s = 0; s < ns; ++s) {
       int64_t n = 1;
       for (int e : J.g.legs[s]) n *= t->rank[e];
       n *= (int64_t)J.pd[s] * J.pd[s];
-      t->dout[s] = J.pd[s];
       total = std::max(total, t->op_offset[s] + n);
     }
     for (int64_t i = 0; i < 2 * total; ++i) need(std::isfinite(op_data[i]), "non-finite TPO element");

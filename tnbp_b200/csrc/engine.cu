@@ -1382,7 +1382,7 @@ static int launch_batch_t(const SweepBatch& b, cudaStream_t stream) {
       }
       case SweepLaunch::GRAM_CORE:
         if constexpr (sizeof(R) == 4)
-          k_gram<R><<<(unsigned)L.nblocks, kThreads, 0, stream>>>(static_cast<const GramTask*>(tasks), begins, L.ntask);
+          k_gram<<<(unsigned)L.nblocks, kThreads, 0, stream>>>(static_cast<const GramTask*>(tasks), begins, L.ntask);
         break;
       case SweepLaunch::MSG:
         k_msg_finalize<R, MR><<<L.ntask, kFinalizeThreads, 0, stream>>>(static_cast<const MsgTask*>(tasks));
@@ -2169,7 +2169,7 @@ void Job::env_grams(const std::vector<EnvReq>& reqs, DevBuf& out, std::vector<si
   if (!gt.empty()) {
     prepare_kernels(sprec);
     if (sprec == TNBP_C128) (launch_gram_f64(static_cast<GramTask*>(dgt.p), static_cast<long long*>(dgb.p), (int)gt.size(), nb, stream), note_launch());
-    else (k_gram<float><<<(unsigned)nb, kThreads, 0, stream>>>(static_cast<GramTask*>(dgt.p), static_cast<long long*>(dgb.p), (int)gt.size()), note_launch());
+    else (k_gram<<<(unsigned)nb, kThreads, 0, stream>>>(static_cast<GramTask*>(dgt.p), static_cast<long long*>(dgb.p), (int)gt.size()), note_launch());
     CK(cudaGetLastError());
     (k_partial_sum<<<(unsigned)pt.size(), kThreads, 0, stream>>>(static_cast<PartialSumTask*>(dpt.p)), note_launch());
     CK(cudaGetLastError());

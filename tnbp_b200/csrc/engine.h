@@ -173,7 +173,6 @@ void check_tc_error(cudaStream_t stream);
 struct Tpo {
   std::vector<int> rank;          // per edge
   std::vector<int64_t> op_offset; // per site, complex elements
-  std::vector<int> dout;          // per site
   DevBuf ops;
   ~Tpo();
 };

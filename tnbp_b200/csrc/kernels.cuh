@@ -161,10 +161,10 @@ struct GramTask {
   int f64 = 0;            // complex128 operands
 };
 
-template <typename R>
-__global__ void __launch_bounds__(kThreads) k_gram(const GramTask* __restrict__ tasks,
-                                                   const long long* __restrict__ begins, int ntask) {
-  using C = typename cvec<R>::type;
+// complex64; the complex128 ones run k_gram_f64 (dmma.cuh).
+static __global__ void __launch_bounds__(kThreads) k_gram(const GramTask* __restrict__ tasks,
+                                                          const long long* __restrict__ begins, int ntask) {
+  using C = float2;
   // rows padded to 34 elements: 16-byte aligned pairs for the 2x2 tiles
   __shared__ __align__(16) C As[kRowTile][kColTile + 2];
   __shared__ __align__(16) C Bs[kRowTile][kColTile + 2];
@@ -182,10 +182,8 @@ __global__ void __launch_bounds__(kThreads) k_gram(const GramTask* __restrict__ 
   const C* B = static_cast<const C*>(tk.B);
   const long long L = tk.L, LD = tk.L * tk.D, LDM = tk.L * tk.D * tk.M;
   const bool qfast = L >= kRowTile;
-  // complex64: each 32-row tile is summed in FP32 and added to an FP64
-  // accumulator, so rounding does not grow with the chunk length (up to 4096
-  // rows); complex128 accumulates directly.
-  constexpr bool kPromote = sizeof(R) == 4;
+  // each 32-row tile is summed in FP32 and added to an FP64 accumulator, so
+  // rounding does not grow with the chunk length (up to 16384 rows)
   const int ga0 = 2 * (threadIdx.x % 16), gb0 = 2 * (threadIdx.x / 16);
   C acc[4];
   double2 accd[4];
@@ -221,21 +219,19 @@ __global__ void __launch_bounds__(kThreads) k_gram(const GramTask* __restrict__ 
       cfma_conj(acc[2], x0, y1);
       cfma_conj(acc[3], x1, y1);
     }
-    if (kPromote) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const double2 t = to_d2(acc[i]);
-        accd[i].x += t.x;
-        accd[i].y += t.y;
-        acc[i] = czero<C>();
-      }
+    for (int i = 0; i < 4; ++i) {
+      const double2 t = to_d2(acc[i]);
+      accd[i].x += t.x;
+      accd[i].y += t.y;
+      acc[i] = czero<C>();
     }
   }
   double2* part = tk.partial + (long long)chunk * tk.C * tk.C;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int a = ca0 + ga0 + (i & 1), bb = cb0 + gb0 + (i >> 1);
-    if (a < tk.C && bb < tk.C) part[a + (long long)tk.C * bb] = kPromote ? accd[i] : to_d2(acc[i]);
+    if (a < tk.C && bb < tk.C) part[a + (long long)tk.C * bb] = accd[i];
   }
 }
 

@@ -157,14 +157,13 @@ std::shared_ptr<const TpoSet> Server::tpo_set(
   std::vector<tnbp_host::Layer> layers;
   build(ts->edges, layers);
   if (ts->edges.empty()) throw Error(TNBP_EINVAL, "the circuit has no two-qubit gate (no edges)");
-  const size_t ne = ts->edges.size(), ns = tnbp_host::site_labels(ts->edges).size();
+  const size_t ne = ts->edges.size();
   ts->rank_max.assign(ne, 1);
   for (const auto& L : layers) {
     auto t = std::make_unique<Tpo>();
     t->rank.assign(L.edge_rank.begin(), L.edge_rank.end());
     for (size_t e = 0; e < ne; ++e) ts->rank_max[e] = std::max(ts->rank_max[e], t->rank[e]);
     t->op_offset = L.op_offset;
-    t->dout.assign(ns, 2);
     t->ops.alloc(L.op_data.size() * sizeof(double), stream);
     CK(cudaMemcpyAsync(t->ops.p, L.op_data.data(), L.op_data.size() * sizeof(double), cudaMemcpyHostToDevice,
                        stream));

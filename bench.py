@@ -615,7 +615,7 @@ def run_ours(args, rank, world, local_rank):
         "higher_is_better": True,
         "scaling": "weak",
         "vs_baseline": None,
-        "dtype": "mixed: c64 BP sweeps (3xTF32 / FP32 products, FP64 sums) on a c128 state; FP64 absorb, "
+        "dtype": "mixed: c64 BP sweeps (3xTF32 / FP32 products, FP64 sums; c128 at bonds up to 8) on a c128 state; FP64 absorb, "
                  "truncation, measurement",
         "data": "synthetic (seeded kicked-Ising circuit and Pauli observable)",
         "config": workload_config(theta_h, world),
@@ -642,8 +642,8 @@ def run_ours(args, rank, world, local_rank):
                         "hbm_achieved_gbs": (tot_by / n_sw) / ((tot_ms / n_sw) / 1e3) / 1e9 if n_sw else None,
                         "hbm_peak_gbs": peaks.get("hbm_gbs")},
     }
-    # the DRAM bytes that the sweep's schedule moves at D = 32 (computed, see
-    # the file) over the measured sweep time: how close the kernels run to the
+    # the DRAM bytes that a sweep moves at D = 32 (counters, scaled: see the
+    # file) over the measured sweep time: how close the kernels run to the
     # copy bandwidth on the traffic they must move
     if traffic and n_sw and peaks.get("hbm_gbs"):
         rate = traffic / ((tot_ms / n_sw) / 1e3) / 1e9

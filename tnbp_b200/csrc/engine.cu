@@ -729,7 +729,7 @@ void Job::autotune_waves() {
 // matters, but sweeps that a program counts itself may run on messages far
 // from any fixed point, where loopy BP amplifies rounding (random states: 600
 // to 1000 times in four sweeps).  Their results do not depend on how fast a
-// loop is.  36 sites at D = 32, d = 2, per sweep: 5.8 ms leg by leg, 2.4 ms in
+// loop is.  36 sites at D = 32, d = 2, per sweep: 6.0 ms leg by leg, 2.9 ms in
 // pairs.  A program that changes between the two keeps both plans and their
 // graphs (building one takes the host longer than most sweeps), as long as
 // the shared scratch does not move and the budget holds both.

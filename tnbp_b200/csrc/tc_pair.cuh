@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(tc::kPairThreads, 1)
 // Why: two launches of the leg kernel read and wrote the tensor twice; here it
 // is read and written once, which leaves HBM (64 KB per tile at D = 32, about
 // 2800 cycles per SM) and the two products' MMAs (1700 cycles) as bounds.
-// One 8x8 sweep at D = 32: 1.86 ms in the leg kernel, 0.88 ms here (5400
+// One sweep of an 8x8 lattice's loop at D = 32: 1.86 ms in the leg kernel, 0.88 ms here (5400
 // cycles per tile when planes are contiguous, 8000 when memory runs along o
 // and a tile is 32-byte pieces); 6x6 at D = 16: 0.09 -> 0.04 ms.
 //

@@ -57,11 +57,12 @@ with tb.State(EDGES, tb.MIXED) as st:
 """
 
 
-def test_changing_between_loops_and_single_sweeps_keeps_both_plans():
+@pytest.mark.parametrize("wave_mb", ["0", "1"])  # one wave, several
+def test_changing_between_loops_and_single_sweeps_keeps_both_plans(wave_mb):
     if not tb.device_available():
         pytest.fail("no CUDA device: the GPU tests need a B200")
     code = SCRIPT.format(root=ROOT, oracle=os.path.join(ROOT, "oracle"), tests=os.path.join(ROOT, "tests"))
-    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, TNBP_TRACE="1"), capture_output=True, text=True, timeout=300)
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, TNBP_TRACE="1", TNBP_WAVE_MB=wave_mb), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
     builds = [int(l.split()[1]) for l in r.stderr.splitlines() if l.split()[:1] == ["sweep.build_plan"]]
     # one more at most: the second plan may need a larger scratch than the first was built on

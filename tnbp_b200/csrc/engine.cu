@@ -805,7 +805,7 @@ void Job::build_plan(bool loop) {
     TNBP_TRACE_SCOPE("sweep.build_plan.scratch_limit");
     cap = slots <= ws_scratch.bytes ? whole : scratch_limit();
   }
-  const size_t budget = wave_budget && wave_budget < cap ? wave_budget : cap;
+  const size_t wave_bytes = wave_budget && wave_budget < cap ? wave_budget : cap;
   std::vector<std::vector<int>> waves;
   {
     size_t bytes = 0;
@@ -814,7 +814,7 @@ void Job::build_plan(bool loop) {
       const Unit& U = units[i];
       const size_t site_b = slot_bytes(U);
       const size_t add = (size_t)U.nbuf * site_b + (U.site == last_site ? 0 : site_b);
-      if (waves.empty() || (budget && bytes + add > budget && !waves.back().empty())) {
+      if (waves.empty() || (wave_bytes && bytes + add > wave_bytes && !waves.back().empty())) {
         waves.emplace_back();
         bytes = site_b + (size_t)U.nbuf * site_b;
       } else {
